@@ -1450,7 +1450,7 @@ PYRB_API pyrb_result pyrb_path_edit(const pyrb_exec* e, uint64_t nodes, uint64_t
         prim_tile[j] = uint32_t(pt);
         // attribute slots of the job's target (32-bit values, or 8 indices per word)
         at += (uint64_t(jb.attr_count) + jb.edit_count + kPeTile - 1) / kPeTile;
-        pt += (uint64_t(jb.prim_count) + kBlock - 1) / kBlock;
+        pt += (uint64_t(jb.prim_count) + kPeBoxWarps - 1) / kPeBoxWarps;
     }
     attr_tile[count] = uint32_t(at);
     prim_tile[count] = uint32_t(pt);
@@ -1499,10 +1499,11 @@ PYRB_API pyrb_result pyrb_path_edit(const pyrb_exec* e, uint64_t nodes, uint64_t
     if (err == cudaSuccess)
         err = cudaMemcpyAsync(plan + count + 1, prim_tile.data(), uint64_t(count + 1) * 4, cudaMemcpyHostToDevice, st);
     if (err != cudaSuccess) return done(fail(PYRB_ERROR_CUDA, "path edit upload: %s", cudaGetErrorString(err)));
-    const size_t ops_smem = size_t(max_edits) * 16;
-    cudaFuncSetAttribute(k_path_attrs, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kPeMaxEdits * 16));
-    launch(k_path_walk, (count + 3) / 4, 128, 0, st, p);
-    if (at) launch(k_path_attrs, uint32_t(at), kBlock, ops_smem, st, p);
+    launch(k_path_walk, count, 32, 0, st, p);
+    if (at) {
+        launch(k_path_map, count, kBlock, size_t(max_edits) * sizeof(uint2), st, p);
+        launch(k_path_attrs, uint32_t(at), kBlock, 0, st, p);
+    }
     if (pt) launch(k_path_boxes, uint32_t(pt), kBlock, 0, st, p);
     err = cudaGetLastError();
     if (err == cudaSuccess) err = cudaMemcpyAsync(jobs, p.jobs, jobs_bytes, cudaMemcpyDeviceToHost, st);

@@ -34,6 +34,21 @@ __device__ __forceinline__ uint32_t upper_index(const uint32_t* arr, uint32_t n,
     return lo;
 }
 
+// The same by a whole warp: 32 probes a round trip instead of one.
+template <typename T>
+__device__ __forceinline__ uint32_t warp_upper_index(const T* arr, uint32_t n, T v) {
+    const unsigned lane = threadIdx.x & 31;
+    uint32_t lo = 0;
+    while (n > 1) {
+        const uint32_t step = (n + 31) / 32;
+        const bool le = lane * step < n && __ldg(arr + lo + lane * step) <= v;
+        const uint32_t k = 31 - __clz(__ballot_sync(kFull, le) | 1u);
+        lo += k * step;
+        n = min(step, n - k * step);
+    }
+    return lo;
+}
+
 __device__ __forceinline__ uint32_t dyn_tile(uint32_t* counters, uint32_t ctr, uint32_t* s_slot) {
     if (threadIdx.x == 0) *s_slot = atomicAdd(counters + kCtrTiles + ctr, 1u);
     __syncthreads();

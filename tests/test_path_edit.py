@@ -208,3 +208,58 @@ def test_cuda_path_edit_matches_oracle(palette):
     assert np.array_equal(da.cpu().numpy().view(np.uint32), a2)
     assert np.array_equal(dp.cpu().numpy().reshape(-1, 16), p2)
     assert np.array_equal(db.cpu().numpy().reshape(-1).view(np.uint32), b2.reshape(-1).view(np.uint32))
+
+
+def _decode(keys):
+    """Coordinates of sorted voxel keys (brick Morton << 6 | x&3 + 4(y&3) + 16(z&3))."""
+    k = keys.astype(np.uint64)
+    out = np.empty((len(k), 3), np.uint32)
+    for a in range(3):
+        v = (k >> np.uint64(2 * a)) & np.uint64(3)
+        for b in range(18):
+            v |= ((k >> np.uint64(6 + 3 * b + a)) & np.uint64(1)) << np.uint64(2 + b)
+        out[:, a] = v
+    return out
+
+
+# The attribute rewrite takes tiles of 4096 attributes and traces every operation once:
+# operations at the tiles' first and last places, voxels set, removed and set again in one
+# job, the most edits a job takes, more prims than the walk keeps in shared memory, and
+# one prim over the whole volume.
+@pytest.mark.gpu
+@pytest.mark.parametrize("log2,rt,n_edits,kind", [(6, 6, 96, "edges"), (6, 3, 300, "edges"), (5, 5, 4096, "repeats"),
+                                                  (7, 3, 400, "random")])
+def test_cuda_path_edit_tiles_and_repeats(log2, rt, n_edits, kind):
+    import torch
+    from pyrit_b200 import gpu_build, native
+    from gpu_helpers import dev
+    rng = np.random.default_rng(log2 * 100 + rt)
+    vox, g = _geometry(log2, rt, 60 + log2)
+    ed = _edits(rng, log2, vox, n_edits)
+    if kind == "edges":
+        ranks = np.concatenate([np.arange(t - 2, t + 3) for t in range(4096, g.voxel_count, 4096)] +
+                               [np.array([0, 1, g.voxel_count - 1])])
+        pos = _decode(g.keys[ranks[ranks < g.voxel_count]])
+        at = rng.permutation(n_edits)[:min(len(pos), n_edits)]
+        ed[at, :3] = pos[:len(at)]
+        ed[at, 3] = np.where(rng.random(len(at)) < 0.6, 0, 9)
+    elif kind == "repeats":
+        ed[:, :3] = ed[rng.integers(0, 200, n_edits), :3]
+    job = _job(g, log2, rt, n_edits)
+    nodes = np.concatenate([g.nodes, np.zeros(job["node_cap"], np.uint32)])
+    leaves = np.concatenate([g.leaves, np.zeros(job["leaf_cap"], np.uint64)])
+    attrs = np.concatenate([g.attrs, np.zeros(job["attr_cap"], np.uint32)])
+    n2, l2, a2, p2, b2, want = orc.path_edit(nodes, leaves, attrs, [job], ed, g.prims, g.aabbs)
+    dn, dl, da = dev(nodes), dev(leaves), dev(attrs)
+    dp, db = torch.from_numpy(g.prims.copy()).cuda(), torch.from_numpy(g.aabbs.copy()).cuda()
+    j = native.PathEditJob(**job)
+    j.prims, j.aabbs = dp.data_ptr(), db.data_ptr()
+    out = [j]
+    gpu_build.path_edit(dn, dl, da, out, ed)
+    assert (out[0].out_root, out[0].out_count, out[0].out_flags) == tuple(
+        want[0][k] for k in ("out_root", "out_count", "out_flags"))
+    assert np.array_equal(dn.cpu().numpy().view(np.uint32), n2)
+    assert np.array_equal(dl.cpu().numpy().view(np.uint64), l2)
+    assert np.array_equal(da.cpu().numpy().view(np.uint32), a2)
+    assert np.array_equal(dp.cpu().numpy().reshape(-1), p2.reshape(-1))
+    assert np.array_equal(db.cpu().numpy().reshape(-1).view(np.uint32), b2.reshape(-1).view(np.uint32))
