@@ -1387,7 +1387,7 @@ PYRB_API pyrb_result pyrb_palette_scan(const pyrb_exec* e, uint64_t attrs, const
     CU(cudaMemsetAsync(tab, 0xFF, uint64_t(count) * kPalSlots * 8, st));
     CU(cudaMemsetAsync(small, 0, uint64_t(count) * 4, st));
     launch(k_pal_collect, j.tiles, kBlock, 0, st, j.p);
-    launch(k_pal_layout, (count + kBlock - 1) / kBlock, kBlock, 0, st, j.p);
+    launch(k_pal_layout, (count + kWarps - 1) / kWarps, kBlock, 0, st, j.p);
     CU(cudaGetLastError());
     CU(cudaMemcpyAsync(counts, j.p.counts, uint64_t(count) * 4, cudaMemcpyDeviceToHost, st));
     CU(cudaStreamSynchronize(st));

@@ -2172,15 +2172,17 @@ __global__ void __launch_bounds__(32) k_selftest_wait(uint64_t* status, uint32_t
 // The reference runs one CTA per chunk and inserts values into a 64-slot shared
 // table in whatever order its threads arrive; the palette is the table's slot order.
 // Here chunks are cut into tiles of kPalTile voxels over the whole GPU: each tile
-// collects its distinct values with the first voxel index of each (warp match_any,
-// then a shared table), merges them into the chunk's global table (value, first
-// index by atomicMin), and one thread per chunk then inserts the values in order of
+// collects its distinct values with the first voxel index of each (every thread skips
+// the values it met last, the others go to a shared table), merges them into the
+// chunk's global table (value, first index by atomicMin), and one warp per chunk then
+// inserts the values in order of
 // first occurrence into the reference's 64-slot table (same hash, linear probing)
 // to lay out the palette: the order the reference produces when its inserts arrive
 // in voxel order, which is every order when no two values share a home slot.
 // ---------------------------------------------------------------------------
 constexpr uint32_t kPalSlots = 64, kPalMax = 16, kPalEmpty = 0xFFFFFFFFu, kPalOverflow = 0xFFFFFFFFu;
-constexpr uint32_t kPalTile = 4096;
+constexpr uint32_t kPalSteps = 4;
+constexpr uint32_t kPalTile = 4096 * kPalSteps;  // voxels per block
 
 struct PaletteDesc {
     const uint32_t* attrs;
@@ -2202,17 +2204,21 @@ __device__ __forceinline__ uint32_t pal_hash(uint32_t v) {  // palette.zig:34-38
     return h ^ (h >> 15);
 }
 
-// Insert (v, idx) into a kPalSlots table (shared or global); returns false when full.
-__device__ __forceinline__ bool pal_insert(uint32_t* vals, uint32_t* firsts, uint32_t v, uint32_t idx) {
+// Insert (v, idx) into a kPalSlots table (shared or global); returns false when full, *fresh
+// says whether the value was new.
+// A value that is there with an index at least as small needs no atomic (an atomic takes
+// its turn with all others on its address, and most inserts are of known values).
+__device__ __forceinline__ bool pal_insert(uint32_t* vals, uint32_t* firsts, uint32_t v, uint32_t idx, bool* fresh) {
     uint32_t s = pal_hash(v) & (kPalSlots - 1);
     for (uint32_t probes = 0; probes < kPalSlots; ++probes) {
-        uint32_t cur = atomicAdd(vals + s, 0u);
+        uint32_t cur = *reinterpret_cast<volatile uint32_t*>(vals + s);
         if (cur == kPalEmpty) {
             cur = atomicCAS(vals + s, kPalEmpty, v);
+            *fresh = cur == kPalEmpty;
             if (cur == kPalEmpty) cur = v;
         }
         if (cur == v) {
-            atomicMin(firsts + s, idx);
+            if (*reinterpret_cast<volatile uint32_t*>(firsts + s) > idx) atomicMin(firsts + s, idx);
             return true;
         }
         s = (s + 1) & (kPalSlots - 1);
@@ -2220,123 +2226,196 @@ __device__ __forceinline__ bool pal_insert(uint32_t* vals, uint32_t* firsts, uin
     return false;
 }
 
-__device__ __forceinline__ uint32_t pal_chunk_of(const PaletteDesc& p, uint32_t tile) {
-    return upper_index(p.tile_of, p.count + 1, tile);
+// A step's kPalPer rows of kBlock attributes, all loads in flight. A block takes four
+// steps, since its look-ups before the first and its merge after the last are round
+// trips: scan + pack of 200 M attributes in 256 chunks take 691 / 614 / 568 us a call with
+// one / two / four (1208 when every row went through match_any, which costs some hundred
+// cycles where a row holds more than a few values, and every word's 8 attributes through
+// 16 comparisons each). Now the kernels take 180 and 221 us: the attributes' 0.8 GB are
+// 125 us at the copy rate, the pack writes another 0.25 GB.
+constexpr uint32_t kPalStep = kPalTile / kPalSteps, kPalPer = kPalStep / kBlock;
+__device__ __forceinline__ void pal_load(const uint32_t* attrs, uint32_t n, uint32_t (&v)[kPalPer]) {
+#pragma unroll
+    for (uint32_t k = 0; k < kPalPer; ++k) {
+        const uint32_t i = k * kBlock + threadIdx.x;
+        v[k] = i < n ? __ldg(attrs + i) : kPalEmpty;
+    }
 }
 
 __global__ void __launch_bounds__(kBlock) k_pal_collect(PaletteDesc p) {
     grid_dep_wait();
-    __shared__ uint32_t s_val[kPalSlots], s_first[kPalSlots];
-    __shared__ uint32_t s_full;
+    __shared__ uint32_t s_val[kPalSlots], s_first[kPalSlots], s_found;
     const uint32_t tile = blockIdx.x;
-    if (tile >= p.tile_of[p.count]) return;
-    const uint32_t c = pal_chunk_of(p, tile);
-    const uint32_t lo = p.first[c] + (tile - p.tile_of[c]) * kPalTile;
-    const uint32_t hi = min(p.first[c + 1], lo + kPalTile);
     if (threadIdx.x < kPalSlots) {
         s_val[threadIdx.x] = kPalEmpty;
         s_first[threadIdx.x] = 0xFFFFFFFFu;
     }
-    if (threadIdx.x == 0) s_full = 0;
+    if (threadIdx.x == 0) s_found = 0;
+    const uint32_t c = warp_upper_index(p.tile_of, p.count + 1, tile);
+    if (c >= p.count) return;
+    const uint32_t lo = __ldg(p.first + c) + (tile - __ldg(p.tile_of + c)) * kPalTile;
+    const uint32_t hi = min(__ldg(p.first + c + 1), lo + kPalTile);
+    // (a chunk that another tile found to hold too many values: nothing more to learn)
+    if (*reinterpret_cast<volatile uint32_t*>(p.gflag + c) != 0) return;
+    uint32_t v[kPalPer];
+    pal_load(p.attrs + lo, hi - lo, v);
     __syncthreads();
+    // A thread passes over the two values it met last. Of the others in a row of the warp
+    // each value is inserted once, by its lowest lane: a thread's rows and a row's lanes are
+    // in index order, so the smallest index of a value is among the inserted ones.
+    // (0xFFFFFFFF is the table's empty marker and never enters a palette, as in the
+    // reference.)
     const unsigned lane = threadIdx.x & 31;
-    for (uint32_t base = lo; base < hi; base += kBlock) {
-        const uint32_t i = base + threadIdx.x;
-        const bool in = i < hi;
-        const uint32_t v = in ? __ldg(p.attrs + i) : 0u;
-        // one insert per distinct value of the warp, by its lowest lane (smallest index)
-        const unsigned peers = __match_any_sync(kFull, in ? v : kPalEmpty);
-        // (0xFFFFFFFF is the table's empty marker and never enters a palette, as in the reference)
-        if (in && v != kPalEmpty && lane == unsigned(__ffs(peers) - 1)) {
-            if (!pal_insert(s_val, s_first, v, i)) s_full = 1;
+    uint32_t last0 = kPalEmpty, last1 = kPalEmpty;
+    for (uint32_t base = lo; base < hi; base += kPalStep) {
+        if (base != lo) pal_load(p.attrs + base, hi - base, v);
+#pragma unroll
+        for (uint32_t k = 0; k < kPalPer; ++k) {
+            const uint32_t x = v[k];
+            const bool need = x != kPalEmpty && x != last0 && x != last1;
+            unsigned todo = __ballot_sync(kFull, need);
+            if (!todo) continue;
+            // (more values than a palette holds: nothing more to learn)
+            if (*reinterpret_cast<volatile uint32_t*>(&s_found) > kPalMax) break;
+            while (todo) {
+                const uint32_t lead = __ffs(todo) - 1;
+                todo &= ~__ballot_sync(kFull, x == __shfl_sync(kFull, x, lead));
+                bool fresh = false;
+                if (lane == lead && (!pal_insert(s_val, s_first, x, base + k * kBlock + threadIdx.x, &fresh) || fresh))
+                    atomicAdd(&s_found, 1u);
+            }
+            if (need) {
+                last1 = last0;
+                last0 = x;
+            }
         }
+        if (*reinterpret_cast<volatile uint32_t*>(&s_found) > kPalMax) break;
     }
     __syncthreads();
-    if (s_full) {
+    if (s_found > kPalMax) {  // the chunk keeps its 32-bit attributes
         if (threadIdx.x == 0) atomicOr(p.gflag + c, 1u);
         return;
     }
     if (threadIdx.x < kPalSlots && s_val[threadIdx.x] != kPalEmpty) {
+        bool fresh;
         if (!pal_insert(p.gval + uint64_t(c) * kPalSlots, p.gfirst + uint64_t(c) * kPalSlots, s_val[threadIdx.x],
-                        s_first[threadIdx.x]))
+                        s_first[threadIdx.x], &fresh))
             atomicOr(p.gflag + c, 1u);
     }
 }
 
+// One warp per chunk: the chunk's values in order of first occurrence into the
+// reference's table, then the palette in its slot order.
 __global__ void __launch_bounds__(kBlock) k_pal_layout(PaletteDesc p) {
     grid_dep_wait();
-    const uint32_t c = blockIdx.x * kBlock + threadIdx.x;
+    __shared__ uint32_t s_v[kWarps][kPalMax], s_f[kWarps][kPalMax], s_key[kWarps][kPalSlots];
+    const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t c = blockIdx.x * kWarps + warp;
     if (c >= p.count) return;
     const uint32_t* gv = p.gval + uint64_t(c) * kPalSlots;
     const uint32_t* gf = p.gfirst + uint64_t(c) * kPalSlots;
-    uint32_t v[kPalMax + 1], f[kPalMax + 1], n = 0;
-    bool over = p.gflag[c] != 0;
-    for (uint32_t s = 0; s < kPalSlots && !over; ++s) {
-        if (gv[s] == kPalEmpty) continue;
-        if (n == kPalMax) { over = true; break; }
-        // insertion by first occurrence
-        uint32_t k = n++;
-        while (k > 0 && f[k - 1] > gf[s]) { v[k] = v[k - 1]; f[k] = f[k - 1]; --k; }
-        v[k] = gv[s];
-        f[k] = gf[s];
-    }
-    if (over) {
-        p.counts[c] = kPalOverflow;
+    const uint32_t va = gv[lane], vb = gv[lane + 32], fa = gf[lane], fb = gf[lane + 32];
+    const unsigned ha = __ballot_sync(kFull, va != kPalEmpty), hb = __ballot_sync(kFull, vb != kPalEmpty);
+    const uint32_t n = __popc(ha) + __popc(hb);
+    if (p.gflag[c] != 0 || n > kPalMax) {
+        if (lane == 0) p.counts[c] = kPalOverflow;
         return;
     }
-    // the reference's table with the values inserted in that order
-    uint32_t keys[kPalSlots];
-    for (uint32_t s = 0; s < kPalSlots; ++s) keys[s] = kPalEmpty;
+    const unsigned lt = lanemask_lt();
+    uint32_t *v = s_v[warp], *f = s_f[warp], *key = s_key[warp];
+    key[lane] = key[lane + 32] = kPalEmpty;
+    if (va != kPalEmpty) f[__popc(ha & lt)] = fa;
+    if (vb != kPalEmpty) f[__popc(ha) + __popc(hb & lt)] = fb;
+    __syncwarp();
+    // first occurrences are all different: a value's place is the number of smaller ones
+    uint32_t ra = 0, rb = 0;
     for (uint32_t k = 0; k < n; ++k) {
-        uint32_t s = pal_hash(v[k]) & (kPalSlots - 1);
-        while (keys[s] != kPalEmpty) s = (s + 1) & (kPalSlots - 1);
-        keys[s] = v[k];
+        ra += f[k] < fa ? 1u : 0u;
+        rb += f[k] < fb ? 1u : 0u;
     }
+    if (va != kPalEmpty) v[ra] = va;
+    if (vb != kPalEmpty) v[rb] = vb;
+    __syncwarp();
+    if (lane == 0) {
+        for (uint32_t k = 0; k < n; ++k) {
+            uint32_t s = pal_hash(v[k]) & (kPalSlots - 1);
+            while (key[s] != kPalEmpty) s = (s + 1) & (kPalSlots - 1);
+            key[s] = v[k];
+        }
+    }
+    __syncwarp();
+    const uint32_t ka = key[lane], kb = key[lane + 32];
+    const unsigned ma = __ballot_sync(kFull, ka != kPalEmpty), mb = __ballot_sync(kFull, kb != kPalEmpty);
     uint32_t* pal = p.palettes + uint64_t(c) * kPalMax;
-    uint32_t m = 0, p0 = 0;
-    for (uint32_t s = 0; s < kPalSlots; ++s) {
-        if (keys[s] == kPalEmpty) continue;
-        if (m == 0) p0 = keys[s];
-        pal[m++] = keys[s];
-    }
-    for (; m < kPalMax; ++m) pal[m] = n > 0 ? p0 : 0u;
-    p.counts[c] = n;
+    if (ka != kPalEmpty) pal[__popc(ma & lt)] = ka;
+    if (kb != kPalEmpty) pal[__popc(ma) + __popc(mb & lt)] = kb;
+    // padded with the first value
+    const uint32_t p0 = ma ? __shfl_sync(kFull, ka, __ffs(ma) - 1) : mb ? __shfl_sync(kFull, kb, __ffs(mb) - 1) : 0u;
+    if (lane >= n && lane < kPalMax) pal[lane] = p0;
+    if (lane == 0) p.counts[c] = n;
 }
 
-// palette.zig pack: per tile of a chunk, one thread per output word (8 voxels).
+// palette.zig pack: rows of 32 voxels per warp; a voxel's index comes from a table of the
+// palette (or is the thread's last one again), 8 lanes join theirs to a word.
 __global__ void __launch_bounds__(kBlock) k_pal_pack(PaletteDesc p) {
     grid_dep_wait();
-    __shared__ uint32_t s_pal[kPalMax];
+    __shared__ uint32_t s_val[kPalSlots], s_ix[kPalSlots], s_none;
     const uint32_t tile = blockIdx.x;
-    if (tile >= p.tile_of[p.count]) return;
-    const uint32_t c = pal_chunk_of(p, tile);
-    const uint32_t lo = p.first[c], n = p.first[c + 1] - lo;
-    const uint32_t t0 = (tile - p.tile_of[c]) * kPalTile;  // first voxel of the tile within the chunk
+    const uint32_t c = warp_upper_index(p.tile_of, p.count + 1, tile);
+    if (c >= p.count) return;
+    const uint32_t lo = __ldg(p.first + c), n = __ldg(p.first + c + 1) - lo;
+    const uint32_t t0 = (tile - __ldg(p.tile_of + c)) * kPalTile;  // first voxel of the tile within the chunk
     const uint32_t t1 = min(n, t0 + kPalTile);
-    uint32_t* out = p.pool + p.dst[c];
-    if (p.counts[c] == kPalOverflow) {
-        for (uint32_t i = t0 + threadIdx.x; i < t1; i += kBlock) out[i] = __ldg(p.attrs + lo + i);
+    uint32_t* out = p.pool + __ldg(p.dst + c);
+    const bool raw = __ldg(p.counts + c) == kPalOverflow;
+    uint32_t v[kPalPer];
+    pal_load(p.attrs + lo + t0, t1 - t0, v);
+    if (raw) {
+        for (uint32_t base = t0; base < t1; base += kPalStep) {
+            if (base != t0) pal_load(p.attrs + lo + base, t1 - base, v);
+#pragma unroll
+            for (uint32_t k = 0; k < kPalPer; ++k)
+                if (base + k * kBlock + threadIdx.x < t1) out[base + k * kBlock + threadIdx.x] = v[k];
+        }
         return;
     }
+    if (threadIdx.x < kPalSlots) {
+        s_val[threadIdx.x] = kPalEmpty;
+        s_ix[threadIdx.x] = 0xFFFFFFFFu;
+    }
+    if (threadIdx.x == 0) s_none = kPalMax;
+    __syncthreads();
     if (threadIdx.x < kPalMax) {
-        s_pal[threadIdx.x] = p.palettes[uint64_t(c) * kPalMax + threadIdx.x];
-        if (t0 == 0) out[threadIdx.x] = s_pal[threadIdx.x];
+        const uint32_t x = p.palettes[uint64_t(c) * kPalMax + threadIdx.x];
+        if (t0 == 0) out[threadIdx.x] = x;
+        // of equal entries the first; the table's empty marker (in a caller's own palette)
+        // has its index beside the table
+        bool fresh;
+        if (x != kPalEmpty) pal_insert(s_val, s_ix, x, threadIdx.x, &fresh);
+        else atomicMin(&s_none, threadIdx.x);
     }
     __syncthreads();
-    for (uint32_t w = t0 / 8 + threadIdx.x; w < (t1 + 7) / 8; w += kBlock) {
-        uint32_t word = 0;
+    const uint32_t none = s_none < kPalMax ? s_none : 0u;
+    uint32_t last = kPalEmpty, ix = none;
+    for (uint32_t base = t0; base < t1; base += kPalStep) {
+        if (base != t0) pal_load(p.attrs + lo + base, t1 - base, v);
 #pragma unroll
-        for (uint32_t j = 0; j < 8; ++j) {
-            const uint32_t i = w * 8 + j;
-            if (i >= n) break;
-            const uint32_t v = __ldg(p.attrs + lo + i);
-            uint32_t idx = 0;
-#pragma unroll
-            for (int q = kPalMax - 1; q >= 0; --q)
-                if (s_pal[q] == v) idx = uint32_t(q);  // the first equal entry
-            word |= idx << (j * 4);
+        for (uint32_t k = 0; k < kPalPer; ++k) {
+            const uint32_t i = base + k * kBlock + threadIdx.x;
+            if (v[k] != last) {
+                // (a value outside the palette has index 0)
+                last = v[k];
+                ix = last == kPalEmpty ? none : 0u;
+                uint32_t s = pal_hash(last) & (kPalSlots - 1);
+                for (uint32_t key; last != kPalEmpty && (key = s_val[s]) != kPalEmpty; s = (s + 1) & (kPalSlots - 1))
+                    if (key == last) { ix = s_ix[s]; break; }
+            }
+            uint32_t word = i < t1 ? ix << ((threadIdx.x & 7) * 4) : 0u;
+            word |= __shfl_xor_sync(kFull, word, 1);
+            word |= __shfl_xor_sync(kFull, word, 2);
+            word |= __shfl_xor_sync(kFull, word, 4);
+            if ((threadIdx.x & 7) == 0 && i < t1) out[kPalMax + i / 8] = word;
         }
-        out[kPalMax + w] = word;
     }
 }
 

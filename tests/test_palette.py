@@ -103,3 +103,27 @@ def test_palette_of_a_chunk_batch_matches_oracle():
     first = np.array([b.first_voxel[c] for c in nonempty] + [h.voxel_count], np.uint32)
     _check_against_oracle(h.attrs, b.attrs, first)
     b.free()
+
+
+# Blocks of four steps of 4096 voxels: chunks that end around a step's and a block's last
+# voxel, with one value, exactly as many as a palette holds and one more (all of them
+# early, or the last one only at the chunk's end), and the table's empty marker among them.
+@pytest.mark.gpu
+@pytest.mark.parametrize("size", [1, 31, 4095, 4097, 16384, 16385, 40000])
+def test_palette_steps_and_limits(size):
+    from gpu_helpers import dev
+    rng = np.random.default_rng(size)
+    parts = []
+    for k in (1, 2, 16, 17):
+        vals = rng.integers(1, 1 << 31, k, dtype=np.uint64).astype(np.uint32)
+        v = rng.choice(vals, size).astype(np.uint32)
+        parts.append(v)
+        late = rng.choice(vals[:-1] if k > 1 else vals, size).astype(np.uint32)
+        late[-1] = vals[-1]
+        parts.append(late)
+        marked = np.sort(v)          # long runs
+        marked[size // 2] = 0xFFFFFFFF
+        parts.append(marked)
+    first = np.arange(len(parts) + 1, dtype=np.uint32) * size
+    attrs = np.concatenate(parts)
+    _check_against_oracle(attrs, dev(attrs), first)
