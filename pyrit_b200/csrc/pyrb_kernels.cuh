@@ -188,13 +188,13 @@ __global__ void __launch_bounds__(1024) k_plan(BuildDesc d) {
 // ---------------------------------------------------------------------------
 template <typename KeyT>
 __device__ __forceinline__ void encode_voxel(uint4 v, uint32_t log2, uint32_t lb, KeyT& key, uint32_t& val) {
-    const int32_t n = int32_t(1u << log2);
-    int32_t x = int32_t(v.x), y = int32_t(v.y), z = int32_t(v.z);
-    if (x < 0 || y < 0 || z < 0 || x >= n || y >= n || z >= n) {
+    // one test for all axes: a negative coordinate has high bits set, too
+    if ((v.x | v.y | v.z) >> log2) {
         key = KeyT(1) << lb;
         val = 0;
     } else {
-        key = KeyT(voxel_key(uint32_t(x), uint32_t(y), uint32_t(z)));
+        if constexpr (sizeof(KeyT) == 4) key = voxel_key32(v.x, v.y, v.z);
+        else key = KeyT(voxel_key(v.x, v.y, v.z));
         val = v.w;
     }
 }
@@ -229,13 +229,7 @@ __device__ __forceinline__ void load_raw(const BuildDesc& d, uint32_t seg, uint3
             break;
         }
         default: {  // downsample (gbuild.zig:262-274): coarse key of the source voxel
-            uint64_t k = __ldg(d.src_keys + j);
-            uint64_t brick = k >> 6;
-            uint32_t bit = uint32_t(k & 63), sh = d.shift;
-            uint32_t x = ((compact3(brick) << 2) | (bit & 3)) >> sh;
-            uint32_t y = ((compact3(brick >> 1) << 2) | ((bit >> 2) & 3)) >> sh;
-            uint32_t z = ((compact3(brick >> 2) << 2) | (bit >> 4)) >> sh;
-            key = KeyT(voxel_key(x, y, z));
+            key = KeyT(coarse_key(__ldg(d.src_keys + j), d.shift));
             val = __ldg(d.src_vals + j);
             break;
         }

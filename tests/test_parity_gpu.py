@@ -405,3 +405,19 @@ def test_world_edit_overlay_with_repeated_coordinates(gb, seed):
     offs = np.concatenate([[0], np.cumsum([len(sg) for sg in segs])]).astype(np.uint32)
     o = orc.gb_build_chunks(log2, 4, cap2, packed, offs)
     assert_same_build(got, o, chunks=True, label="repeated edits")
+
+
+@pytest.mark.parametrize("n_src", [1, 31, 32, 4097, 20000])
+@pytest.mark.parametrize("shift", [1, 3])
+def test_downsample_rows_of_shared_cells(gb, n_src, shift):
+    """Runs of source voxels that share a coarse cell, cut by the ends of warp rows and of
+    4096-voxel tiles, from full bricks (every neighbour replaced) to single voxels; the
+    source voxel with the largest key gives the attribute."""
+    rng = np.random.default_rng(n_src)
+    idx = np.arange(20000) if n_src > 4097 else np.sort(rng.choice(32 ** 3, n_src, replace=False))
+    pts = np.stack([idx % 32, (idx // 32) % 32, idx // 1024, 1 + idx % 251], 1).astype(np.uint32)
+    src = orc.gb_build(5 if shift == 1 else 6, 3, pts)
+    log2 = 5 if shift == 1 else 6
+    kd, vd = dev(src.keys), dev(src.attrs)
+    g = gb.downsample(log2, 3, kd, vd, src.voxel_count, shift).download()
+    assert_same_build(g, orc.gb_downsample(log2, 3, src.keys, src.attrs, shift), label=f"{n_src} {shift}")
