@@ -425,7 +425,7 @@ struct Plan {
     uint64_t o_table[kMaxLevels + 2] = {}, o_bstat[kMaxLevels + 2] = {}, o_ostat[kMaxLevels + 2] = {};
     uint64_t o_chunk_first = 0, o_roots = 0, o_prim_start = 0, o_seg_entry = 0, o_seg_tile = 0;
     uint64_t o_k0 = 0, o_v0 = 0, o_k1 = 0, o_v1 = 0, o_bkey = 0, o_bmask = 0, o_bfirst = 0, o_bref = 0;
-    uint64_t o_grid = 0, o_grid_off = 0, o_grid_count = 0, o_chunk_vstart = 0, o_grid_super = 0;
+    uint64_t o_grid = 0, o_grid_off = 0, o_grid_count = 0, o_chunk_vstart = 0, o_grid_super = 0, o_grid_scan = 0;
     uint64_t o_bcount = 0, o_brec = 0, o_bloc = 0, o_bsum = 0;
     uint64_t o_set[2][7] = {};
     uint64_t o_cwords = 0, o_binst = 0, o_bdisp = 0;
@@ -621,6 +621,7 @@ pyrb_result plan_build(const Job& job, const Tune* fixed, Plan& p) {
     }
     if (p.grid) p.o_grid = zl.take(grid_cells * 8);
     if (d.grid_fold) p.o_grid_super = zl.take((uint64_t(d.grid_tiles) / 64 + 1) * 8);
+    else if (p.grid || p.bucket) p.o_grid_scan = zl.take((uint64_t(d.grid_tiles) / kGridScanTile + 1) * 8);
     p.zero_bytes = align_up(zl.size, 256);
     Layout fl;  // 0xFF region follows
     fl.size = p.zero_bytes;
@@ -713,6 +714,7 @@ void bind_plan(Plan& p, uint64_t scratch, const uint64_t outs[6], const Job& job
         d.grid_off = static_cast<uint64_t*>(at(p.o_grid_off));
         d.grid_count = static_cast<uint64_t*>(at(p.o_grid_count));
         d.grid_super = static_cast<uint64_t*>(at(p.o_grid_super));
+        d.grid_scan_status = static_cast<uint64_t*>(at(p.o_grid_scan));
         d.chunk_vstart = static_cast<uint32_t*>(at(p.o_chunk_vstart));
     }
     if (p.grid) {
@@ -830,7 +832,7 @@ uint32_t launch_plan(const Plan& p, const std::vector<LevelDesc>& levels, cudaSt
         launch(k_grid_count<true>, d.grid_tiles, kBlock, 0, st, d);
         prof.mark("bucket_tile_count");
         if (!d.grid_fold) {
-            launch(k_grid_scan, 1, kGridScanThreads, 0, st, d);
+            launch(k_grid_scan, (d.grid_tiles + kGridScanTile - 1) / kGridScanTile, kBlock, 0, st, d);
             prof.mark("grid_scan");
         }
         launch(k_grid_write<true>, d.grid_tiles, kBlock, 0, st, d);
@@ -847,7 +849,7 @@ uint32_t launch_plan(const Plan& p, const std::vector<LevelDesc>& levels, cudaSt
         launch(k_grid_count<false>, d.grid_tiles, kBlock, 0, st, d);
         prof.mark("grid_count");
         if (!d.grid_fold) {
-            launch(k_grid_scan, 1, kGridScanThreads, 0, st, d);
+            launch(k_grid_scan, (d.grid_tiles + kGridScanTile - 1) / kGridScanTile, kBlock, 0, st, d);
             prof.mark("grid_scan");
         }
         launch(k_grid_write<false>, d.grid_tiles, kBlock, 0, st, d);

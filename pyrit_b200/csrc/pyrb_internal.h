@@ -151,6 +151,7 @@ struct BuildDesc {
     uint64_t* grid_off;      // [K + 1] first cell of every chunk (k_plan)
     uint64_t* grid_count;    // [grid_tiles] voxels | bricks << 32 per tile, then their exclusive scan
     uint32_t grid_fold;      // no scan pass (grid_tiles <= kGridFoldTiles): group sums, added up by the write pass
+    uint64_t* grid_scan_status;  // else: look-back status of the scan (zeroed)
     uint64_t* grid_super;    // grid_fold: [grid_tiles / 64 + 1] voxels | bricks << 32 of every 64 tiles (zeroed)
     uint32_t* chunk_vstart;  // [K] voxels before the first cell of every chunk (chunk builds)
 
