@@ -74,10 +74,14 @@ std::atomic<uint32_t> g_load_pct{50};
 // Sort or cell grid for the voxels of a build (pyrb_tuning.path)
 constexpr uint32_t kPathAuto = 0, kPathSort = 1, kPathGrid = 2, kPathBucket = 3;
 std::atomic<uint32_t> g_path{kPathAuto};
-// The grid path is taken automatically while the chunks hold at most this many cells
-// per entry (dense volumes: 256^3 noise at 30 % solid has 3.3, terrain chunks 2), and
-// at most kGridMaxCells cells in all (8 B each).
-constexpr uint64_t kGridCellsPerEntry = 4;
+// The grid path is taken automatically while the chunks hold at most 4 cells per entry
+// (dense volumes: 256^3 noise at 30 % solid has 3.3, terrain chunks 2) or 2^23 cells more
+// than that, and at most kGridMaxCells cells in all (8 B each). The bytes of a grid of 2^23
+// cells stay in the L2, and the sort's passes have a floor of some 80 us however few the
+// entries are: a 128^3 scene of 295,000 voxels (7 cells per entry) orders in 35 us on the
+// grid, 92 sorted; beyond both terms the cells' traffic loses (1024^3 at 15 %, 6.6 cells
+// per entry: 9.3 ms against 5.3).
+constexpr uint64_t kGridCellsPerEntry = 4, kGridFreeCells = uint64_t(1) << 23;
 // A node level takes tiles of one item per thread below this many large tiles (2 per SM)
 constexpr uint32_t kSmallLevelTiles = 296;
 constexpr uint64_t kGridMaxCells = uint64_t(1) << 33;
@@ -504,7 +508,7 @@ pyrb_result plan_build(const Job& job, const Tune* fixed, Plan& p) {
     uint64_t grid_cells = 0;
     for (uint32_t l = 3; l <= log2 && !p.key64; ++l) grid_cells += per_log2[l] << (3 * l);
     if (!p.key64 && grid_cells <= kGridMaxCells)
-        p.grid = path == kPathGrid || (path == kPathAuto && grid_cells <= kGridCellsPerEntry * nmax);
+        p.grid = path == kPathGrid || (path == kPathAuto && grid_cells <= kGridCellsPerEntry * nmax + kGridFreeCells);
     if (!p.key64 && !p.grid && (grid_cells >> 6) <= kBucketMaxBricks)
         p.bucket = path == kPathBucket;
     if (p.grid || p.bucket) tile_keys = 4096;  // the scatter's tiles over the entries
@@ -1643,10 +1647,15 @@ PYRB_API pyrb_result pyrb_build_noalloc(void* stream, uint32_t log2_size, uint32
     j.rt_req = rt_log2_req;
     j.voxels = edits;
     j.n_new = n_new;
-    // one fixed tuning: the scratch bound below holds for it at every allowed size
-    const Tune fixed{8, 4096, 50, kPathSort};
+    // one fixed tuning: the scratch bound below holds for the sort at every allowed size;
+    // the grid where it fits, too (edges up to 2^7)
+    const Tune fixed{8, 4096, 50, kPathAuto}, sorted{8, 4096, 50, kPathSort};
     Plan p;
     pyrb_result r = plan_build(j, &fixed, p);
+    if (r == PYRB_OK && p.scratch_bytes > kStaticScratchBytes) {
+        p = Plan();
+        r = plan_build(j, &sorted, p);
+    }
     if (r != PYRB_OK) return r;
     const uint32_t prim_need = std::max(p.d.prim_bound, 1u);
     if (node_capacity < p.d.node_bound || leaf_capacity < p.B || voxel_capacity < p.nmax || prim_capacity < prim_need)
