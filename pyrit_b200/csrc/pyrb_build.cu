@@ -589,6 +589,7 @@ pyrb_result plan_build(const Job& job, const Tune* fixed, Plan& p) {
     d.prim_bound = P[rt - 1];
     if (p.grid || p.bucket) {
         d.use_grid = p.grid ? 1u : 0u;
+        d.one_seg = p.grid && (job.mode == kModePlain || job.mode == kModeDownsample) ? 1u : 0u;
         d.use_bucket = p.bucket ? 1u : 0u;
         d.grid_cells = grid_cells;
         d.grid_tiles = uint32_t(std::max<uint64_t>((grid_cells + 64 * kGridTileBricks - 1) / (64 * kGridTileBricks), 1));
@@ -820,9 +821,11 @@ uint32_t launch_plan(const Plan& p, const std::vector<LevelDesc>& levels, cudaSt
     if (*err != cudaSuccess) return 0;
     prof.mark("memset");
     uint32_t launches = 0;
-    launch(k_plan, 1, 1024, 0, st, d);
-    ++launches;
-    prof.mark("plan");
+    if (!d.one_seg) {
+        launch(k_plan, 1, 1024, 0, st, d);
+        ++launches;
+        prof.mark("plan");
+    }
     if ((*err = cudaGetLastError()) != cudaSuccess) return 0;
     if (p.bucket) {
         launch(k_bkt_count, d.sort_tiles, kBlock, 0, st, d);

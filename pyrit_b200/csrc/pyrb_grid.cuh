@@ -46,10 +46,21 @@ __device__ __forceinline__ void red_max_u64(uint64_t* p, uint64_t v) {
 // keys and downsampling) take the fast loop: the chunk's voxel and edit lists are
 // resolved once per tile, and each thread keeps kScatterBatch 16-byte loads in flight
 // before it encodes them.
+// A single volume is one stretch of entries: no plan to look anything up in.
+__device__ __forceinline__ TileSpan grid_span(const BuildDesc& d, uint32_t tile) {
+    if (!d.one_seg) return tile_span(d, tile);
+    TileSpan t;
+    t.seg = 0;
+    t.first_tile = 0;
+    t.start = tile * d.tile_keys;
+    t.count = t.start < d.n_total ? min(d.tile_keys, d.n_total - t.start) : 0u;
+    return t;
+}
+
 constexpr int kScatterBatch = 4;
 template <typename F>
 __device__ __forceinline__ void for_tile_entries(const BuildDesc& d, const TileSpan& sp, F&& f) {
-    const uint32_t seg_begin = __ldg(d.seg_entry + sp.seg);
+    const uint32_t seg_begin = d.one_seg ? 0u : __ldg(d.seg_entry + sp.seg);
     const uint32_t inv = 1u << d.lb;
     // the segment's entries: src[0, nv) then esrc[0, ...)
     const uint4* src = nullptr;
@@ -149,22 +160,12 @@ __device__ __forceinline__ void for_tile_entries(const BuildDesc& d, const TileS
 __global__ void __launch_bounds__(kBlock) k_grid_scatter(BuildDesc d) {
     grid_dep_wait();
     const uint32_t tile = blockIdx.x;
-    if (tile >= d.seg_tile[d.seg_count]) return;
-    const TileSpan sp = tile_span(d, tile);
-    uint64_t* cells = d.grid + __ldg(d.grid_off + sp.seg);
+    if (!d.one_seg && tile >= d.seg_tile[d.seg_count]) return;
+    const TileSpan sp = grid_span(d, tile);
+    uint64_t* cells = d.grid + (d.one_seg ? 0 : __ldg(d.grid_off + sp.seg));
     for_tile_entries(d, sp, [&](uint32_t e, uint32_t key, uint32_t val) {
         red_max_u64(cells + key, (uint64_t(e + 1) << 32) | val);
     });
-}
-
-// Chunk holding cell `cell` (grid_off non-decreasing, grid_off[0] = 0 <= cell).
-__device__ __forceinline__ uint32_t grid_chunk(const BuildDesc& d, uint64_t cell) {
-    uint32_t lo = 0, hi = d.seg_count;
-    while (hi - lo > 1) {
-        const uint32_t mid = (lo + hi) >> 1;
-        if (__ldg(d.grid_off + mid) <= cell) lo = mid; else hi = mid;
-    }
-    return lo;
 }
 
 // The attribute words of a warp's kGridWarpBricks bricks: cells lane and 32 + lane of
@@ -417,9 +418,9 @@ __global__ void __launch_bounds__(kBlock, 5) k_grid_write(BuildDesc d) {
     uint32_t vpos = uint32_t(wofs), bpos = uint32_t(wofs >> 32);
     const unsigned lt = lanemask_lt();
     uint32_t seg = 0;
-    uint64_t seg_lo = 0, seg_hi = 0;
-    if (wb0 < nbricks) {
-        seg = grid_chunk(d, wb0 << 6);
+    uint64_t seg_lo = 0, seg_hi = d.grid_cells;
+    if (wb0 < nbricks && !d.one_seg) {
+        seg = warp_upper_index(d.grid_off, d.seg_count, uint64_t(wb0) << 6);
         seg_lo = __ldg(d.grid_off + seg);
         seg_hi = __ldg(d.grid_off + seg + 1);
     }

@@ -145,6 +145,7 @@ struct BuildDesc {
     // ends up holding the last entry of its position. Replaces the sort and the
     // unique pass: a streaming compaction of the cells gives the sorted unique voxels.
     uint32_t use_grid;
+    uint32_t one_seg;        // grid of a single volume: one segment, no plan kernel
     uint32_t grid_tiles;     // compaction tiles of kGridTileBricks bricks
     uint64_t grid_cells;     // cells of all chunks (a multiple of 64)
     uint64_t* grid;          // [grid_cells], zeroed before the build

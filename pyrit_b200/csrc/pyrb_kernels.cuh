@@ -82,10 +82,7 @@ __device__ __forceinline__ uint32_t dyn_tile_and(uint32_t* counters, uint32_t ct
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(1024) k_plan(BuildDesc d) {
     grid_dep_wait();
-    __shared__ uint32_t s_scan[2][1024];
-    __shared__ uint32_t s_carry[2];
-    __shared__ uint64_t s_cells[1024];
-    __shared__ uint64_t s_cell_carry;
+    __shared__ uint64_t s_warp[2][32];
     const uint32_t K = d.seg_count;
     if (K == 1 && d.mode != kModeChunksEdits) {
         // one segment (a single volume): no scans
@@ -108,8 +105,8 @@ __global__ void __launch_bounds__(1024) k_plan(BuildDesc d) {
         }
         return;
     }
-    if (threadIdx.x == 0) { s_carry[0] = 0; s_carry[1] = 0; s_cell_carry = 0; }
-    __syncthreads();
+    const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint64_t carry = 0, cell_carry = 0;  // entries | tiles << 31 (both below 2^31), cells
     for (uint32_t base = 0; base < K; base += 1024) {
         uint32_t c = base + threadIdx.x;
         uint32_t size = 0;
@@ -135,49 +132,42 @@ __global__ void __launch_bounds__(1024) k_plan(BuildDesc d) {
                 default: size = d.n_total; break;
             }
         }
-        uint32_t tiles = (size + d.tile_keys - 1) / d.tile_keys;
-        s_scan[0][threadIdx.x] = size;
-        s_scan[1][threadIdx.x] = tiles;
-        __syncthreads();
-        // inclusive Hillis-Steele scan of both arrays
-        for (uint32_t o = 1; o < 1024; o <<= 1) {
-            uint32_t a = threadIdx.x >= o ? s_scan[0][threadIdx.x - o] : 0;
-            uint32_t b = threadIdx.x >= o ? s_scan[1][threadIdx.x - o] : 0;
-            __syncthreads();
-            s_scan[0][threadIdx.x] += a;
-            s_scan[1][threadIdx.x] += b;
-            __syncthreads();
+        const uint64_t both = size | uint64_t((size + d.tile_keys - 1) / d.tile_keys) << 31;
+        // first cell of every chunk in the cell grid (chunk after chunk)
+        uint64_t cells = 0;
+        if ((d.use_grid | d.use_bucket) && c < K)
+            cells = uint64_t(1) << (3 * (d.mode == kModeBatch ? __ldg(d.chunk_log2 + c) : d.log2));
+        // inclusive scans: in the warp, then over the warps' totals by every warp
+        uint64_t x = both, y = cells;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint64_t a = __shfl_up_sync(kFull, x, o), b = __shfl_up_sync(kFull, y, o);
+            if (lane >= unsigned(o)) { x += a; y += b; }
         }
+        if (lane == 31) { s_warp[0][warp] = x; s_warp[1][warp] = y; }
+        __syncthreads();
+        uint64_t tx = s_warp[0][lane], ty = s_warp[1][lane];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint64_t a = __shfl_up_sync(kFull, tx, o), b = __shfl_up_sync(kFull, ty, o);
+            if (lane >= unsigned(o)) { tx += a; ty += b; }
+        }
+        const uint64_t px = __shfl_sync(kFull, tx, (warp + 31) & 31), py = __shfl_sync(kFull, ty, (warp + 31) & 31);
+        x += carry + (warp ? px : 0) - both;
+        y += cell_carry + (warp ? py : 0) - cells;
         if (c < K) {
-            d.seg_entry[c] = s_carry[0] + s_scan[0][threadIdx.x] - size;
-            d.seg_tile[c] = s_carry[1] + s_scan[1][threadIdx.x] - tiles;
+            d.seg_entry[c] = uint32_t(x & 0x7FFFFFFFu);
+            d.seg_tile[c] = uint32_t(x >> 31);
+            if (d.use_grid | d.use_bucket) d.grid_off[c] = y;
         }
-        if (d.use_grid | d.use_bucket) {
-            // first cell of every chunk in the cell grid (chunk after chunk)
-            const uint32_t l = c < K ? (d.mode == kModeBatch ? __ldg(d.chunk_log2 + c) : d.log2) : 0;
-            const uint64_t cells = c < K ? uint64_t(1) << (3 * l) : 0;
-            s_cells[threadIdx.x] = cells;
-            __syncthreads();
-            for (uint32_t o = 1; o < 1024; o <<= 1) {
-                const uint64_t a = threadIdx.x >= o ? s_cells[threadIdx.x - o] : 0;
-                __syncthreads();
-                s_cells[threadIdx.x] += a;
-                __syncthreads();
-            }
-            if (c < K) d.grid_off[c] = s_cell_carry + s_cells[threadIdx.x] - cells;
-        }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            s_carry[0] += s_scan[0][1023];
-            s_carry[1] += s_scan[1][1023];
-            if (d.use_grid | d.use_bucket) s_cell_carry += s_cells[1023];
-        }
-        __syncthreads();
+        carry += __shfl_sync(kFull, tx, 31);
+        cell_carry += __shfl_sync(kFull, ty, 31);
+        __syncthreads();  // s_warp is written again
     }
     if (threadIdx.x == 0) {
-        d.seg_entry[K] = s_carry[0];
-        d.seg_tile[K] = s_carry[1];
-        if (d.use_grid | d.use_bucket) d.grid_off[K] = s_cell_carry;
+        d.seg_entry[K] = uint32_t(carry & 0x7FFFFFFFu);
+        d.seg_tile[K] = uint32_t(carry >> 31);
+        if (d.use_grid | d.use_bucket) d.grid_off[K] = cell_carry;
     }
 }
 
