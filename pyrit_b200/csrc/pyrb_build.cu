@@ -851,7 +851,13 @@ uint32_t launch_plan(const Plan& p, const std::vector<LevelDesc>& levels, cudaSt
             ++launches;
         }
     } else if (p.grid) {
-        launch(k_grid_scatter, d.sort_tiles, kBlock, 0, st, d);
+        if (d.one_seg && d.n_old) {
+            launch(k_grid_old, (d.n_old + 8 * kBlock - 1) / (8 * kBlock), kBlock, 0, st, d);
+            prof.mark("grid_old");
+            ++launches;
+        }
+        launch(k_grid_scatter, d.one_seg ? std::max((d.n_total - d.n_old + d.tile_keys - 1) / d.tile_keys, 1u) : d.sort_tiles,
+               kBlock, 0, st, d);
         prof.mark("grid_scatter");
         launch(k_grid_count<false>, d.grid_tiles, kBlock, 0, st, d);
         prof.mark("grid_count");

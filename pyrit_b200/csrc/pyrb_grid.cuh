@@ -52,7 +52,7 @@ __device__ __forceinline__ TileSpan grid_span(const BuildDesc& d, uint32_t tile)
     TileSpan t;
     t.seg = 0;
     t.first_tile = 0;
-    t.start = tile * d.tile_keys;
+    t.start = d.n_old + tile * d.tile_keys;  // (old entries go to the grid by themselves)
     t.count = t.start < d.n_total ? min(d.tile_keys, d.n_total - t.start) : 0u;
     return t;
 }
@@ -69,7 +69,7 @@ __device__ __forceinline__ void for_tile_entries(const BuildDesc& d, const TileS
     bool fast = true;
     switch (d.mode) {
         case kModePlain:
-            fast = d.n_old == 0;
+            fast = d.n_old == 0 || d.one_seg;
             src = d.voxels;
             nv = d.n_new;
             break;
@@ -94,7 +94,7 @@ __device__ __forceinline__ void for_tile_entries(const BuildDesc& d, const TileS
             fast = false;
             break;
     }
-    const uint32_t j0 = sp.start - seg_begin;
+    const uint32_t j0 = sp.start - seg_begin - (d.one_seg ? d.n_old : 0u);
     if (d.mode == kModeDownsample) {
         const unsigned lane = threadIdx.x & 31;
         for (uint32_t base = 0; base < sp.count; base += kScatterBatch * kBlock) {
@@ -154,6 +154,27 @@ __device__ __forceinline__ void for_tile_entries(const BuildDesc& d, const TileS
             if (idx < sp.count && !(key & inv)) f(sp.start + idx, key, val);
         }
     }
+}
+
+// Old entries of a plain build -> cells. Their keys are sorted and unique and every entry
+// after them overrides them, so they are stored, before the others' atomics: the stores
+// are neighbours, while an atomic takes the L2 as long for each of their sectors as for
+// one on its own (5 M old voxels and 90,000 edits: 39 us by atomics, 21 like this).
+__global__ void __launch_bounds__(kBlock) k_grid_old(BuildDesc d) {
+    grid_dep_wait();
+    constexpr int kBatch = 8;
+    const uint32_t e0 = blockIdx.x * kBatch * kBlock + threadIdx.x;
+    uint64_t key[kBatch];
+    uint32_t val[kBatch];
+#pragma unroll
+    for (int k = 0; k < kBatch; ++k) {
+        const uint32_t e = e0 + k * kBlock;
+        key[k] = e < d.n_old ? __ldcs(d.old_keys + e) : ~0ull;
+        val[k] = e < d.n_old ? __ldcs(d.old_vals + e) : 0u;
+    }
+#pragma unroll
+    for (int k = 0; k < kBatch; ++k)
+        if (key[k] < d.grid_cells) d.grid[key[k]] = uint64_t(e0 + k * kBlock + 1) << 32 | val[k];
 }
 
 // Entries -> cells: an atomic max of (entry index + 1) << 32 | value.

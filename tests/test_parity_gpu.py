@@ -421,3 +421,19 @@ def test_downsample_rows_of_shared_cells(gb, n_src, shift):
     kd, vd = dev(src.keys), dev(src.attrs)
     g = gb.downsample(log2, 3, kd, vd, src.voxel_count, shift).download()
     assert_same_build(g, orc.gb_downsample(log2, 3, src.keys, src.attrs, shift), label=f"{n_src} {shift}")
+
+
+@pytest.mark.parametrize("n_old,n_new", [(1, 1), (2047, 3), (2048, 4096), (2049, 4097), (9000, 0), (9000, 500)])
+def test_old_voxels_and_edits_at_tile_edges(gb, n_old, n_new):
+    """Old voxels (stored by themselves) around the edges of their tiles, edits that set,
+    change and delete old and new positions, repeat them and lie outside the volume."""
+    rng = np.random.default_rng(n_old + n_new)
+    cells = np.sort(rng.choice(32 ** 3, n_old, replace=False))
+    pts = np.stack([cells % 32, (cells // 32) % 32, cells // 1024, 1 + cells % 7], 1).astype(np.uint32)
+    old = orc.gb_build(5, 3, pts)
+    ed = np.concatenate([rng.integers(0, 33, (n_new, 3)), rng.integers(0, 5, (n_new, 1))], 1).astype(np.uint32)
+    if n_new > 2:
+        ed[::3, :3] = pts[rng.integers(0, n_old, len(ed[::3])), :3]
+    g = gb.build(5, 3, dev(ed) if n_new else None, old_keys=dev(old.keys), old_vals=dev(old.attrs),
+                 n_old=n_old).download()
+    assert_same_build(g, orc.gb_build(5, 3, ed, old_keys=old.keys, old_vals=old.attrs), label=f"{n_old}+{n_new}")
