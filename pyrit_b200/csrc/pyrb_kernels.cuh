@@ -1767,9 +1767,38 @@ __global__ void __launch_bounds__(kBlock) k_prims(BuildDesc d, LevelDesc L) {
 // ---------------------------------------------------------------------------
 constexpr uint32_t kTailPer = kTailMaxChildren / kTailThreads;  // children (and parents) per thread
 constexpr uint32_t kTailScanWords = 72;
+// Levels with at most kTailSmall parents keep these in shared memory too (records, words
+// and a table of their own), one per thread: nothing of such a level waits for a global
+// round trip but the staging of the first. Both kinds share the space behind the children.
+constexpr uint32_t kTailSmall = 1024, kTailSmallSlots = 2048;
+constexpr size_t kTailBigBytes = size_t(kTailMaxChildren) * (4 + 2 + 1) + size_t(kTailSlots) * (4 + 4);
+constexpr size_t kTailSmallBytes = size_t(kTailSmall) * (kNodeStride * 4 + 4 + 4 + 4 + 2) + size_t(kTailSmallSlots) * (4 + 4);
 constexpr size_t tail_smem_bytes() {
-    return size_t(kTailMaxChildren) * (8 + 8 + 8 + 4 + 4 + 4 + 2 + 1) + size_t(kTailSlots) * (4 + 4) +
-           kTailScanWords * 4;
+    return size_t(kTailMaxChildren) * (8 + 8 + 8 + 4 + 4) + kTailScanWords * 4 +
+           (kTailBigBytes > kTailSmallBytes ? kTailBigBytes : kTailSmallBytes);
+}
+
+// Exclusive scan over the block with one barrier: every warp scans the warp sums itself.
+// sm: 32 words that are not written again before every thread has passed another barrier.
+__device__ __forceinline__ uint32_t tail_scan1(uint32_t v, uint32_t* sm, uint32_t* total) {
+    const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t x = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(kFull, x, o);
+        if (lane >= unsigned(o)) x += y;
+    }
+    if (lane == 31) sm[warp] = x;
+    __syncthreads();
+    uint32_t w = sm[lane];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(kFull, w, o);
+        if (lane >= unsigned(o)) w += y;
+    }
+    *total = __shfl_sync(kFull, w, 31);
+    const uint32_t before = __shfl_sync(kFull, w, (warp + 31) & 31);
+    return (warp ? before : 0u) + x - v;
 }
 
 __device__ __forceinline__ uint32_t tail_scan(uint32_t v, uint32_t* sm, uint32_t* total) {
@@ -1811,6 +1840,33 @@ __device__ __forceinline__ void tail_words(const uint32_t* words, uint32_t q, ui
     }
 }
 
+// Prim q of the RT level: a parent's cell, box, first voxel and node; prev: the key of the
+// parent before it.
+__device__ __forceinline__ void tail_prim(const BuildDesc& d, uint32_t q, uint64_t full, uint64_t plo, uint64_t phi,
+                                          uint32_t pfirst, uint32_t node, uint64_t prev, uint32_t local_shift) {
+    const uint64_t key = full & ((1ull << local_shift) - 1);
+    const uint32_t chunk = uint32_t(full >> local_shift);
+    const uint32_t first = d.chunked ? d.chunk_first[chunk] : 0;
+    const uint32_t cx = compact3(key), cy = compact3(key >> 1), cz = compact3(key >> 2);
+    const uint32_t size = 1u << d.rt_log2;
+    uint4 rec;
+    rec.x = node;
+    rec.y = pfirst - first;
+    const uint64_t pc = pack_cell(cx, cy, cz);
+    rec.z = uint32_t(pc);
+    rec.w = uint32_t(pc >> 32);
+    reinterpret_cast<uint4*>(d.prims)[q] = rec;
+    const float eps = 1.0f / 256.0f;
+    float* b = d.aabbs + uint64_t(q) * 6;
+    b[0] = __fsub_rn(__fadd_rn(float(cx * size), float(cell_x(plo))), eps);
+    b[1] = __fsub_rn(__fadd_rn(float(cy * size), float(cell_y(plo))), eps);
+    b[2] = __fsub_rn(__fadd_rn(float(cz * size), float(cell_z(plo))), eps);
+    b[3] = __fadd_rn(__fadd_rn(float(cx * size), float(cell_x(phi))), eps);
+    b[4] = __fadd_rn(__fadd_rn(float(cy * size), float(cell_y(phi))), eps);
+    b[5] = __fadd_rn(__fadd_rn(float(cz * size), float(cell_z(phi))), eps);
+    if (d.chunked && (q == 0 || (prev >> local_shift) != chunk)) d.prim_start[chunk] = q;
+}
+
 __global__ void __launch_bounds__(kTailThreads) k_tail(BuildDesc d, TailDesc T) {
     grid_dep_wait();
     extern __shared__ uint64_t tsm64[];
@@ -1819,12 +1875,21 @@ __global__ void __launch_bounds__(kTailThreads) k_tail(BuildDesc d, TailDesc T) 
     uint64_t* shi = slo + kTailMaxChildren;
     uint32_t* sref = reinterpret_cast<uint32_t*>(shi + kTailMaxChildren);
     uint32_t* scnt = sref + kTailMaxChildren;
-    uint32_t* pval = scnt + kTailMaxChildren;                          // parent: hash, then (owners) node offset
+    uint32_t* scan = scnt + kTailMaxChildren;
+    // a level of many parents
+    uint32_t* pval = scan + kTailScanWords;                            // parent: hash, then (owners) node offset
     uint32_t* tkey = pval + kTailMaxChildren;                          // table: parent index + 1
     uint32_t* towner = tkey + kTailSlots;                              // table: minimum parent index
-    uint32_t* scan = towner + kTailSlots;
-    uint16_t* pslot = reinterpret_cast<uint16_t*>(scan + kTailScanWords);  // parent -> slot
+    uint16_t* pslot = reinterpret_cast<uint16_t*>(towner + kTailSlots);    // parent -> slot
     uint8_t* plen = reinterpret_cast<uint8_t*>(pslot + kTailMaxChildren);  // parent -> words
+    // a level of at most kTailSmall parents
+    uint32_t* mwords = scan + kTailScanWords;                          // [kTailSmall][kNodeStride]
+    uint32_t* mhash = mwords + kTailSmall * kNodeStride;               // parent: hash, then (owners) node offset
+    uint32_t* mfirst = mhash + kTailSmall;                             // first voxels of the children in shared memory
+    uint32_t* mlen = mfirst + kTailSmall;
+    uint32_t* mkey = mlen + kTailSmall;                                // table: parent index + 1
+    uint32_t* mowner = mkey + kTailSmallSlots;                         // table: minimum parent index
+    uint16_t* mhead = reinterpret_cast<uint16_t*>(mowner + kTailSmallSlots);  // parent -> first child
     static_assert(kTailSlots <= 65536 && kNodeStride < 256, "slot and length fit their arrays");
     __shared__ uint32_t s_cursor, s_children;
     const uint32_t tid = threadIdx.x;
@@ -1834,9 +1899,10 @@ __global__ void __launch_bounds__(kTailThreads) k_tail(BuildDesc d, TailDesc T) 
         s_children = lv0 == 2 ? min(d.counters[kCtrBricks], d.brick_bound)
                               : min(d.counters[kCtrParents + lv0 - 1], T.parent_bound[lv0 - 1]);
     }
-    for (uint32_t i = tid; i < kTailSlots; i += kTailThreads) { tkey[i] = 0; towner[i] = 0xFFFFFFFFu; }
     __syncthreads();
     const uint32_t local_shift = 3 * (d.log2 - d.rt_log2);
+    bool staged = false;  // the children are in shared memory: the parents of a small level
+    uint32_t root_node = 0;
     for (uint32_t lv = lv0; lv < d.log2; ++lv) {
         const uint32_t C = min(s_children, kTailMaxChildren);
         const RecordSet& ps = T.set[(lv - 2) & 1];
@@ -1844,7 +1910,8 @@ __global__ void __launch_bounds__(kTailThreads) k_tail(BuildDesc d, TailDesc T) 
         const bool box = lv + 1 <= d.rt_log2;
         const uint32_t child_size = 1u << lv;
         // 1. stage children (coalesced: child tid + k * kTailThreads)
-        if (lv == 2) {
+        if (staged) {
+        } else if (lv == 2) {
             uint64_t key[kTailPer], mask[kTailPer];
             uint32_t ref[kTailPer], own[kTailPer];
 #pragma unroll
@@ -1912,7 +1979,132 @@ __global__ void __launch_bounds__(kTailThreads) k_tail(BuildDesc d, TailDesc T) 
             if (i < C && (i == 0 || (skey[i] >> 3) != (skey[i - 1] >> 3))) { hmask |= 1u << k; ++hc; }
         }
         uint32_t P;
-        uint32_t pbase = tail_scan(hc, scan, &P);
+        uint32_t pbase = tail_scan1(hc, scan, &P);
+        const bool prims = lv + 1 == d.rt_log2;
+        if (P <= kTailSmall) {
+            // ---- at most one parent per thread, all in shared memory
+            for (uint32_t i = tid; i < kTailSmallSlots; i += kTailThreads) { mkey[i] = 0; mowner[i] = 0xFFFFFFFFu; }
+            uint32_t at = pbase;
+#pragma unroll
+            for (uint32_t k = 0; k < kTailPer; ++k)
+                if ((hmask >> k) & 1) mhead[at++] = uint16_t(tid * kTailPer + k);
+            __syncthreads();
+            const bool mine = tid < P;
+            uint64_t pkey = 0;
+            uint32_t first = 0, mask = 0, count = 0, n = 0, hash = 0;
+            uint32_t refs[8];
+            uint32_t lo[3] = {0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu}, hi[3] = {0, 0, 0};
+            if (mine) {
+                const uint32_t i = mhead[tid];
+                first = staged ? mfirst[i] : lv == 2 ? d.bfirst[i] : __ldcg(cs.first + i);
+                pkey = skey[i] >> 3;
+                bool in = true;
+#pragma unroll
+                for (uint32_t k = 0; k < 8; ++k) {
+                    const uint32_t j = i + k;
+                    uint64_t ck = 0;
+                    in = in && j < C;
+                    if (in) {
+                        ck = skey[j];
+                        in = (ck >> 3) == pkey;
+                    }
+                    refs[k] = 0;
+                    if (!in) continue;
+                    const uint32_t idx = uint32_t(ck & 7);
+                    mask |= 1u << idx;
+                    count = sat_add(count, scnt[j]);
+                    refs[k] = sref[j];
+                    n = k + 1;
+                    if (box) {
+                        uint64_t clo = slo[j], chi = shi[j];
+                        if (lv == 2) brick_box(slo[j], clo, chi);
+                        const uint32_t ox = (idx & 1) * child_size, oy = ((idx >> 1) & 1) * child_size,
+                                       oz = (idx >> 2) * child_size;
+                        lo[0] = min(lo[0], cell_x(clo) + ox); hi[0] = max(hi[0], cell_x(chi) + ox);
+                        lo[1] = min(lo[1], cell_y(clo) + oy); hi[1] = max(hi[1], cell_y(chi) + oy);
+                        lo[2] = min(lo[2], cell_z(clo) + oz); hi[2] = max(hi[2], cell_z(chi) + oz);
+                    }
+                }
+                uint32_t* w = mwords + tid * kNodeStride;
+                w[0] = mask;
+                w[1] = count;
+#pragma unroll
+                for (uint32_t k = 0; k < 8; ++k) w[2 + k] = refs[k];  // (0 behind the last)
+                // a 32-bit hash: equality is decided by the words
+                hash = mask * 0x9E3779B1u ^ count;
+#pragma unroll
+                for (uint32_t k = 0; k < 8; ++k) hash = (hash ^ (hash >> 15)) * 0x85EBCA6Bu + refs[k];
+                hash ^= hash >> 16;
+                hash *= 0xC2B2AE35u;
+                hash ^= hash >> 13;
+                mhash[tid] = hash;
+            }
+            __syncthreads();
+            // dedup: the owner is the minimum parent index
+            uint32_t slot = 0;
+            if (mine) {
+                uint32_t probes = 0;
+                for (slot = hash & (kTailSmallSlots - 1); probes < kTailSmallSlots;
+                     ++probes, slot = (slot + 1) & (kTailSmallSlots - 1)) {
+                    const uint32_t cur = atomicCAS(mkey + slot, 0u, tid + 1);
+                    if (cur == 0) break;
+                    if (mhash[cur - 1] != hash) continue;
+                    const uint32_t* w = mwords + (cur - 1) * kNodeStride;
+                    bool same = w[0] == mask && w[1] == count;
+#pragma unroll
+                    for (uint32_t k = 0; k < 8; ++k) same = same && w[2 + k] == refs[k];
+                    if (same) break;
+                }
+                if (probes == kTailSmallSlots) atomicOr(d.counters + kCtrError, kErrTable);
+                atomicMin(mowner + slot, tid);
+            }
+            __syncthreads();
+            const uint32_t owner = mine ? mowner[slot] : 0xFFFFFFFFu;
+            const bool own = mine && owner == tid;
+            uint32_t both;  // words | owners << 16
+            const uint32_t off = (tail_scan1(own ? (2 + n) | 1u << 16 : 0u, scan + 32, &both) & 0xFFFF) + s_cursor;
+            if (own) {
+                mhash[tid] = off;
+                if (uint64_t(off) + 2 + n <= d.node_bound) {
+                    d.nodes[off] = mask;
+                    d.nodes[off + 1] = count;
+#pragma unroll
+                    for (uint32_t k = 0; k < 8; ++k)
+                        if (k < n) d.nodes[off + 2 + k] = refs[k];
+                } else {
+                    atomicOr(d.counters + kCtrError, kErrBound);
+                }
+            }
+            __syncthreads();  // every owner's offset; the children are done with
+            uint32_t node = 0;
+            const uint64_t plo = pack_cell(lo[0], lo[1], lo[2]), phi = pack_cell(hi[0], hi[1], hi[2]);
+            if (mine) {
+                node = mhash[owner];
+                skey[tid] = pkey;
+                sref[tid] = node;
+                scnt[tid] = count;
+                slo[tid] = plo;
+                shi[tid] = phi;
+                mfirst[tid] = first;
+                if (tid == 0) root_node = node;
+                if (lv + 1 == d.log2 && d.chunked && uint32_t(pkey) < d.seg_count) d.roots[uint32_t(pkey)] = node;
+            }
+            if (tid == 0) {
+                d.counters[kCtrParents + lv] = P;
+                d.counters[kCtrUniqueLv + lv] = both >> 16;
+                s_cursor += both & 0xFFFF;
+                d.counters[kCtrCursor + lv + 1] = s_cursor;
+                s_children = P;
+                if (prims) d.counters[kCtrPrims] = P;
+            }
+            staged = true;
+            __syncthreads();
+            if (prims && mine && tid < d.prim_bound)
+                tail_prim(d, tid, pkey, plo, phi, first, node, tid > 0 ? skey[tid - 1] : 0, local_shift);
+            continue;
+        }
+        // ---- more parents than that
+        for (uint32_t i = tid; i < kTailSlots; i += kTailThreads) { tkey[i] = 0; towner[i] = 0xFFFFFFFFu; }
         // 3. build parents: records and words into global memory, hashes into pval
         uint32_t fst[kTailPer];
 #pragma unroll
@@ -2024,7 +2216,6 @@ __global__ void __launch_bounds__(kTailThreads) k_tail(BuildDesc d, TailDesc T) 
             }
         }
         // 6. references for the next level, prims, roots
-        const bool prims = lv + 1 == d.rt_log2;
         for (uint32_t q = tid; q < P; q += kTailThreads) {
             const uint32_t node = pval[towner[pslot[q]]];
             ps.slot[q] = node;
@@ -2032,27 +2223,7 @@ __global__ void __launch_bounds__(kTailThreads) k_tail(BuildDesc d, TailDesc T) 
                 const uint64_t full = __ldcg(ps.key + q), plo = __ldcg(ps.lo + q), phi = __ldcg(ps.hi + q);
                 const uint32_t pfirst = __ldcg(ps.first + q);
                 const uint64_t prev = q > 0 ? __ldcg(ps.key + q - 1) : 0;
-                const uint64_t key = full & ((1ull << local_shift) - 1);
-                const uint32_t chunk = uint32_t(full >> local_shift);
-                const uint32_t first = d.chunked ? d.chunk_first[chunk] : 0;
-                const uint32_t cx = compact3(key), cy = compact3(key >> 1), cz = compact3(key >> 2);
-                const uint32_t size = 1u << d.rt_log2;
-                uint4 rec;
-                rec.x = node;
-                rec.y = pfirst - first;
-                const uint64_t pc = pack_cell(cx, cy, cz);
-                rec.z = uint32_t(pc);
-                rec.w = uint32_t(pc >> 32);
-                reinterpret_cast<uint4*>(d.prims)[q] = rec;
-                const float eps = 1.0f / 256.0f;
-                float* b = d.aabbs + uint64_t(q) * 6;
-                b[0] = __fsub_rn(__fadd_rn(float(cx * size), float(cell_x(plo))), eps);
-                b[1] = __fsub_rn(__fadd_rn(float(cy * size), float(cell_y(plo))), eps);
-                b[2] = __fsub_rn(__fadd_rn(float(cz * size), float(cell_z(plo))), eps);
-                b[3] = __fadd_rn(__fadd_rn(float(cx * size), float(cell_x(phi))), eps);
-                b[4] = __fadd_rn(__fadd_rn(float(cy * size), float(cell_y(phi))), eps);
-                b[5] = __fadd_rn(__fadd_rn(float(cz * size), float(cell_z(phi))), eps);
-                if (d.chunked && (q == 0 || (prev >> local_shift) != chunk)) d.prim_start[chunk] = q;
+                tail_prim(d, q, full, plo, phi, pfirst, node, prev, local_shift);
             }
             if (lv + 1 == d.log2 && d.chunked) {
                 const uint32_t chunk = uint32_t(__ldcg(ps.key + q));
@@ -2060,8 +2231,6 @@ __global__ void __launch_bounds__(kTailThreads) k_tail(BuildDesc d, TailDesc T) 
             }
         }
         __syncthreads();  // every thread is done with the table
-        // clear the table for the next level
-        for (uint32_t i = tid; i < kTailSlots; i += kTailThreads) { tkey[i] = 0; towner[i] = 0xFFFFFFFFu; }
         if (tid == 0) {
             d.counters[kCtrParents + lv] = P;
             d.counters[kCtrUniqueLv + lv] = utotal;
@@ -2076,7 +2245,7 @@ __global__ void __launch_bounds__(kTailThreads) k_tail(BuildDesc d, TailDesc T) 
         // final counts and the empty geometry (gbuild.zig:607-624)
         const uint32_t top_set = (d.log2 - 1 - 2) & 1;
         uint32_t cursor = s_cursor;
-        uint32_t root = s_children > 0 ? __ldcg(T.set[top_set].slot) : 0;
+        uint32_t root = s_children == 0 ? 0u : staged ? root_node : __ldcg(T.set[top_set].slot);
         if (d.counters[kCtrUnique] == 0) {
             if (cursor + 2 <= d.node_bound) {
                 d.nodes[cursor] = 0;
