@@ -266,12 +266,14 @@ uint32_t launch_levels(const BuildDesc& d, const std::vector<LevelDesc>& levels,
         else
             launch(k_node_build<kNBIT>, L.build_tiles, kBlock, node_build_smem_bytes(L.lv == 2), st, d, L);
         prof.mark("node_build", L.lv);
+        launch(k_node_insert, std::max(std::min((L.parent_bound + kBlock - 1) / kBlock, 148u * 8u), 1u), kBlock, 0, st, d, L);
+        prof.mark("node_insert", L.lv);
         if (L.own_it == 1)
             launch(k_node_own<1>, L.own_tiles, kBlock, 0, st, d, L);
         else
             launch(k_node_own<kNodeIT>, L.own_tiles, kBlock, 0, st, d, L);
         prof.mark("node_own", L.lv);
-        launches += 2;
+        launches += 3;
         if (L.lv + 1 == d.rt_log2) {
             launch(k_prims, std::max((L.parent_bound + kBlock - 1) / kBlock, 1u), kBlock, 0, st, d, L);
             prof.mark("prims", L.lv);
@@ -432,7 +434,7 @@ struct Plan {
     uint64_t o_grid = 0, o_grid_off = 0, o_grid_count = 0, o_chunk_vstart = 0, o_grid_super = 0, o_grid_scan = 0;
     uint64_t o_bcount = 0, o_brec = 0, o_bloc = 0, o_bsum = 0;
     uint64_t o_set[2][7] = {};
-    uint64_t o_cwords = 0, o_binst = 0, o_bdisp = 0;
+    uint64_t o_binst = 0, o_bdisp = 0;
     uint64_t zero_bytes = 0, ff_bytes = 0, scratch_bytes = 0;
     // output buffers (bytes): nodes, leaves, keys, attrs, prims, aabbs
     uint64_t out_size[6] = {};
@@ -671,12 +673,6 @@ pyrb_result plan_build(const Job& job, const Tune* fixed, Plan& p) {
         p.o_set[s][5] = ol.take(m * 8);                 // hi
         p.o_set[s][6] = ol.take(m * kNodeStride * 4);   // words
     }
-    // words of the small levels' parents at their first child's index (one buffer,
-    // levels run one after another)
-    uint64_t cw = 0;
-    for (uint32_t lv = 2; lv < log2; ++lv)
-        if (p.bnb[lv] == 1) cw = std::max<uint64_t>(cw, lv == 2 ? B : P[lv - 1]);
-    p.o_cwords = ol.take(std::max<uint64_t>(cw, 1) * kNodeStride * 4);
     p.scratch_bytes = align_up(ol.size, 256);
     const uint64_t prims = std::max(d.prim_bound, 1u);
     const uint64_t outs[6] = {uint64_t(d.node_bound) * 4, uint64_t(B) * 8, uint64_t(nmax) * 8, uint64_t(nmax) * 4,
@@ -786,7 +782,6 @@ void bind_plan(Plan& p, uint64_t scratch, const uint64_t outs[6], const Job& job
         L.plo = static_cast<uint64_t*>(at(p.o_set[ps][4]));
         L.phi = static_cast<uint64_t*>(at(p.o_set[ps][5]));
         L.pwords = static_cast<uint32_t*>(at(p.o_set[ps][6]));
-        L.cwords = static_cast<uint32_t*>(at(p.o_cwords));
         L.ptable = static_cast<uint4*>(at(p.o_table[lv]));
         L.build_status = static_cast<uint64_t*>(at(p.o_bstat[lv]));
         L.own_status = static_cast<uint64_t*>(at(p.o_ostat[lv]));

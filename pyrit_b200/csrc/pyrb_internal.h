@@ -193,13 +193,11 @@ struct LevelDesc {
     uint64_t* pkey;
     uint32_t* pcnt;
     uint32_t* pfirst;
-    uint32_t* pslot;
+    uint32_t* pslot;         // hash of its words (build), then its slot (insert)
     uint64_t* plo;
     uint64_t* phi;
     uint32_t* pwords;        // [parent_bound][10]
-    uint32_t* cwords;        // build_nb == 1: [child_bound][10], words at the first child's index
-                             // (the table key of these levels: the first child's index + 1)
-    uint4* ptable;           // {key + 1, -, ~owner, node offset}; key: parent index, or first child index
+    uint4* ptable;           // {parent index + 1, hash, ~owner, node offset}
     uint64_t* build_status;
     uint64_t* own_status;
 };

@@ -816,7 +816,7 @@ __global__ void __launch_bounds__(kBlock, 5) k_unique(BuildDesc d, uint32_t fin)
 
 // ---------------------------------------------------------------------------
 // Dedup tables. Leaf table slot: {mask lo, mask hi, ~owner, -};
-// node table slot: {key + 1, 0, ~owner, node offset}. ~owner with
+// node table slot: {parent index + 1, hash, ~owner, node offset}. ~owner with
 // atomicMax makes the minimum index the owner on zero-initialised tables.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ void claim_owner(uint4* slot, uint32_t idx) {
@@ -1215,47 +1215,6 @@ __device__ __forceinline__ uint64_t node_hash(uint32_t mask, uint32_t count, con
     return h;
 }
 
-// Insert parent `par` into the level table. Its words are at key_words[key * stride]
-// (stored before this call: the CAS releases them); colliding residents are compared
-// by their words at key_words[(resident key) * stride]. h is the home slot, refs the
-// parent's child references. Returns the slot; the minimum parent index owns it.
-__device__ __forceinline__ uint32_t node_insert(uint4* table, uint32_t cap, const uint32_t* key_words, uint32_t key,
-                                                uint32_t par, uint32_t h, uint32_t mask, uint32_t count,
-                                                const uint32_t (&refs)[8], uint32_t n, uint32_t* err) {
-    for (uint32_t probe = 0; probe < cap; ++probe) {
-        uint32_t* kp = &table[h].x;
-        uint32_t cur = ld_acquire32(kp);
-        if (cur == 0) {
-            // release: our words (stored before this call) are visible with the key
-            cur = cas_acq_rel32(kp, 0u, key + 1);
-            if (cur == 0) {
-                atomicMax(&table[h].z, ~par);  // first of its words: claim without waiting
-                return h;
-            }
-        }
-        // acquired above: the resident's words are visible
-        const uint32_t* ow = key_words + uint64_t(cur - 1) * kNodeStride;
-        uint32_t o[kNodeStride];
-#pragma unroll
-        for (int k = 0; k < int(kNodeStride); k += 2) {
-            uint2 v = __ldcg(reinterpret_cast<const uint2*>(ow + k));
-            o[k] = v.x;
-            o[k + 1] = v.y;
-        }
-        bool same = o[0] == mask && o[1] == count;
-#pragma unroll
-        for (int k = 0; k < 8; ++k)
-            if (uint32_t(k) < n) same = same && o[2 + k] == refs[k];
-        if (same) {
-            claim_owner(table + h, par);
-            return h;
-        }
-        h = (h + 1) & (cap - 1);
-    }
-    atomicOr(err, kErrTable);
-    return 0;
-}
-
 __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
 // Leaf index of brick b: its own (it owns its mask) or its mask's owner's, found
@@ -1318,18 +1277,14 @@ __device__ __forceinline__ NodeParent node_assemble(const LevelDesc& L, const ui
     return q;
 }
 
-// Records of parent `par` (key, count, first voxel, box, table slot and, when asked
-// for, its words).
+// Records of parent `par`: key, count, first voxel, box, hash, words.
 __device__ __forceinline__ void node_store(const LevelDesc& L, uint32_t par, const NodeParent& q, uint64_t pkey,
-                                           uint32_t first, uint32_t slot, bool words) {
-    if (words) {
-        uint32_t* pw = L.pwords + uint64_t(par) * kNodeStride;
-        pw[0] = q.mask;
-        pw[1] = q.count;
+                                           uint32_t first, uint32_t hash) {
+    uint2* pw = reinterpret_cast<uint2*>(L.pwords + uint64_t(par) * kNodeStride);
+    pw[0] = make_uint2(q.mask, q.count);
 #pragma unroll
-        for (uint32_t k = 0; k < 8; ++k)
-            if (k < q.n) pw[2 + k] = q.refs[k];
-    }
+    for (uint32_t k = 0; k < 8; k += 2)
+        if (k < q.n) pw[1 + k / 2] = make_uint2(q.refs[k], q.refs[k + 1]);
     L.pkey[par] = pkey;
     L.pcnt[par] = q.count;
     L.pfirst[par] = first;
@@ -1337,23 +1292,19 @@ __device__ __forceinline__ void node_store(const LevelDesc& L, uint32_t par, con
         L.plo[par] = pack_cell(q.lo[0], q.lo[1], q.lo[2]);
         L.phi[par] = pack_cell(q.hi[0], q.hi[1], q.hi[2]);
     }
-    L.pslot[par] = slot;
+    L.pslot[par] = hash;
 }
 
 // Tile of the node build: kBlock * NB children staged in shared memory (plus a halo
 // of up to 7 children of the tile's last parent), heads found with warp ballots,
-// positions by a look-back scan, then every thread builds parents from shared memory
-// and inserts them into the level's table.
+// positions by a look-back scan, then every thread builds parents from shared memory.
 // Parents per thread of the node-owner kernel and children per thread of the node
 // build: large levels take 8 and 4 (tiles of 2048 parents / 1024 children), levels
 // small enough to leave most SMs idle with those take 1 (tiles of 256), so that their
 // tiles spread over the whole GPU (plan_build picks per level).
 // Small levels (NB == 1) are latency-bound: a global round trip costs about a
-// microsecond, an acquire-release atomic several. There every load of a staging step
-// is in flight together, and each parent (at most one per thread) is assembled before
-// the look-back: its words go to L.cwords at its first child's index (the table key of
-// these levels), so that the release of the insert after the look-back finds them long
-// performed, and its home slot is prefetched into the L2.
+// microsecond. There every load of a staging step is in flight together, and each parent
+// (at most one per thread) is assembled before the look-back.
 constexpr int kNodeIT = 8;
 constexpr int kNodeTile = kBlock * kNodeIT;     // tile of the node-owner kernel (large levels)
 constexpr int kNBIT = 4;
@@ -1509,68 +1460,40 @@ __device__ __forceinline__ void node_build_tile(const BuildDesc& d, const LevelD
         run += __popc(hb[j]);
     }
     __syncthreads();
-    if constexpr (NB == 1) {
-        // the tile's parents, one per thread: assembled, words published at the first
-        // child's index, home slot prefetched, all before the look-back
-        const bool mine = threadIdx.x < total;
-        NodeParent q;
-        uint32_t i = 0, h = 0;
-        if (mine) {
+    // the parents' records and words, with their hashes for the level's table (the
+    // inserts are a kernel of their own: there every parent's words are visible, and a claim
+    // needs no release and a comparison no acquire)
+    auto put = [&](uint32_t par, const NodeParent& q, uint32_t i) {
+        if (par >= L.parent_bound) {
+            atomicOr(d.counters + kCtrError, kErrBound);
+            return;
+        }
+        const uint32_t hash = uint32_t(node_hash(q.mask, q.count, q.refs, q.n));
+        prefetch_l2(&L.ptable[hash & (L.pcap - 1)]);
+        node_store(L, par, q, skey[cpad(i)] >> 3, sfirst[cpad(i)], hash);
+    };
+    NodeParent q;
+    uint32_t i = 0;
+    if constexpr (NB == 1) {  // at most one parent per thread: assembled before the look-back
+        if (threadIdx.x < total) {
             i = shead[threadIdx.x];
             q = node_assemble(L, skey, slo, shi, scnt, sref, i, tn);
-            uint32_t* cw = L.cwords + uint64_t(t0 + i) * kNodeStride;
-            cw[0] = q.mask;
-            cw[1] = q.count;
-#pragma unroll
-            for (uint32_t k = 0; k < 8; ++k)
-                if (k < q.n) cw[2 + k] = q.refs[k];
-            h = uint32_t(node_hash(q.mask, q.count, q.refs, q.n)) & (L.pcap - 1);
-            prefetch_l2(&L.ptable[h]);
         }
-        if (warp == 0) {
-            uint64_t ex = lookback_warp(L.build_status, tile, 0, total, d.counters + kCtrError);
-            if (lane == 0) s_base = ex;
-        }
-        __syncthreads();
-        if (tile == ntiles - 1 && threadIdx.x == 0) d.counters[kCtrParents + L.lv] = uint32_t(s_base + total);
-        if (mine) {
-            const uint32_t par = uint32_t(s_base) + threadIdx.x;
-            if (par >= L.parent_bound) {
-                atomicOr(d.counters + kCtrError, kErrBound);
-            } else {
-                // the insert first: its release then covers only the words stored above
-                const uint32_t slot = node_insert(L.ptable, L.pcap, L.cwords, t0 + i, par, h, q.mask, q.count,
-                                                  q.refs, q.n, d.counters + kCtrError);
-                node_store(L, par, q, skey[cpad(i)] >> 3, sfirst[cpad(i)], slot, true);
-            }
-        }
+    }
+    if (warp == 0) {
+        uint64_t ex = lookback_warp(L.build_status, tile, 0, total, d.counters + kCtrError);
+        if (lane == 0) s_base = ex;
+    }
+    __syncthreads();
+    if (tile == ntiles - 1 && threadIdx.x == 0) d.counters[kCtrParents + L.lv] = uint32_t(s_base + total);
+    const uint32_t base = uint32_t(s_base);
+    if constexpr (NB == 1) {
+        if (threadIdx.x < total) put(base + threadIdx.x, q, i);
     } else {
-        if (warp == 0) {
-            uint64_t ex = lookback_warp(L.build_status, tile, 0, total, d.counters + kCtrError);
-            if (lane == 0) s_base = ex;
-        }
-        __syncthreads();
-        if (tile == ntiles - 1 && threadIdx.x == 0) d.counters[kCtrParents + L.lv] = uint32_t(s_base + total);
-        const uint32_t base = uint32_t(s_base);
         for (uint32_t hh = threadIdx.x; hh < total; hh += kBlock) {
-            const uint32_t i = shead[hh];
-            const uint32_t par = base + hh;
-            const NodeParent q = node_assemble(L, skey, slo, shi, scnt, sref, i, tn);
-            if (par >= L.parent_bound) {
-                atomicOr(d.counters + kCtrError, kErrBound);
-                continue;
-            }
-            // words first (the insert's release publishes them with the key)
-            uint32_t* pw = L.pwords + uint64_t(par) * kNodeStride;
-            pw[0] = q.mask;
-            pw[1] = q.count;
-#pragma unroll
-            for (uint32_t k = 0; k < 8; ++k)
-                if (k < q.n) pw[2 + k] = q.refs[k];
-            const uint32_t h = uint32_t(node_hash(q.mask, q.count, q.refs, q.n)) & (L.pcap - 1);
-            const uint32_t slot = node_insert(L.ptable, L.pcap, L.pwords, par, par, h, q.mask, q.count, q.refs,
-                                              q.n, d.counters + kCtrError);
-            node_store(L, par, q, skey[cpad(i)] >> 3, sfirst[cpad(i)], slot, false);
+            i = shead[hh];
+            q = node_assemble(L, skey, slo, shi, scnt, sref, i, tn);
+            put(base + hh, q, i);
         }
     }
 }
@@ -1583,6 +1506,69 @@ __global__ void __launch_bounds__(kBlock, NB == 1 ? 6 : 5) k_node_build(BuildDes
     const uint32_t ci = L.lv == 2 ? kCtrBricks : kCtrParents + L.lv - 1;
     const uint32_t tile = dyn_tile_and(d.counters, L.tile_ctr_build, ci, ci, s_tile, &children, &unused);
     node_build_tile<NB>(d, L, tile, children);
+}
+
+// The parents of a level into its table: {index + 1, hash, ~owner, -}, equal words -> same
+// slot, the minimum parent index owns it. An empty slot is claimed with index, hash and
+// ~index in one 16-byte compare-and-swap. The words of every resident were written by the
+// kernel before, so nothing here needs an acquire or a release; they are compared where the
+// hashes are equal. Build, insert and owners of 256^3
+// noise take 18 + 12 + 13 us at level 2 (28,000 parents) and 11 + 10 + 11 at level 3 (4096);
+// with acquire-release inserts in the build kernel 32 + 15 and 32 + 11.
+constexpr int kProbes = 4;
+__global__ void __launch_bounds__(kBlock) k_node_insert(BuildDesc d, LevelDesc L) {
+    grid_dep_wait();
+    const uint32_t P = min(__ldcg(d.counters + kCtrParents + L.lv), L.parent_bound), cmask = L.pcap - 1;
+    for (uint32_t par = blockIdx.x * kBlock + threadIdx.x; par < P; par += gridDim.x * kBlock) {
+        const uint32_t hash = __ldcg(L.pslot + par);
+        uint32_t h = hash & cmask, w[kNodeStride];
+        const uint2* pw = reinterpret_cast<const uint2*>(L.pwords + uint64_t(par) * kNodeStride);
+#pragma unroll
+        for (int k = 0; k < int(kNodeStride); k += 2) {
+            const uint2 v = __ldcg(pw + k / 2);
+            w[k] = v.x;
+            w[k + 1] = v.y;
+        }
+        const uint32_t n = __popc(w[0]);
+        const uint64_t me = uint64_t(hash) << 32 | (par + 1);
+        // slot `at`, last seen as cur: whether the parent ends there
+        auto take = [&](uint32_t at, uint64_t cur) -> bool {
+            uint4* slot = L.ptable + at;
+            if (cur == 0) {
+                uint64_t hi;
+                cas128(slot, 0, 0, me, uint64_t(~par), cur, hi);
+                if (cur == 0) return true;
+            }
+            if (uint32_t(cur >> 32) != hash) return false;
+            const uint2* rw = reinterpret_cast<const uint2*>(L.pwords + uint64_t(uint32_t(cur) - 1) * kNodeStride);
+            bool same = true;
+#pragma unroll
+            for (int k = 0; k < int(kNodeStride); k += 2) {
+                const uint2 v = __ldcg(rw + k / 2);
+                same = same && (uint32_t(k) >= 2 + n || v.x == w[k]) && (uint32_t(k) + 1 >= 2 + n || v.y == w[k + 1]);
+            }
+            if (same) claim_owner(slot, par);
+            return same;
+        };
+        // the home slot by itself (repeated words mostly end there), then kProbes together:
+        // the longest of some thousand sequences (10 to 20 slots at half load) would be a
+        // chain of round trips that the whole level waits for
+        bool done = take(h, ld_relaxed(reinterpret_cast<const uint64_t*>(L.ptable + h)));
+        for (uint32_t probe = 1; probe <= cmask && !done; probe += kProbes) {
+            uint64_t c[kProbes];
+#pragma unroll
+            for (int q = 0; q < kProbes; ++q)
+                c[q] = ld_relaxed(reinterpret_cast<const uint64_t*>(L.ptable + ((hash + probe + q) & cmask)));
+#pragma unroll
+            for (int q = 0; q < kProbes; ++q) {
+                if (done) continue;
+                h = (hash + probe + q) & cmask;
+                done = take(h, c[q]);
+            }
+        }
+        L.pslot[par] = h;
+        if (!done) atomicOr(d.counters + kCtrError, kErrTable);
+    }
 }
 
 // Owners of level lv get word offsets (scan of their lengths) and write their words.
