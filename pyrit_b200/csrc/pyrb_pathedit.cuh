@@ -13,7 +13,7 @@
 // through the root, but a node's words, its children's counts and the prims are read
 // and written by the lanes together), the attribute map (one CTA per job), the attribute
 // rewrite (over the whole GPU) and the boxes (one warp per prim). Every result equals the
-// reference's job by job. 256 jobs of 32 edits over 200 M attributes: 1.11 ms a call, of
+// reference's job by job. 256 jobs of 32 edits over 200 M attributes: 0.86 ms a call, of
 // which the attributes' 1.6 GB take 0.25 at the copy rate; 7.24 with a lane per walk and
 // prim and with every attribute traced through all of its job's operations.
 #pragma once
@@ -48,7 +48,9 @@ struct RtPrim {  // types.zig:518-525
 constexpr uint32_t kPeOpNone = 0, kPeOpSet = 1, kPeOpInsert = 2, kPeOpRemove = 3;
 constexpr uint32_t kPeRebuild = 0x1, kPeEmpty = 0x2, kPeOverflow = 0x4, kPeGrew = 0x8;
 constexpr uint32_t kPeMaxEdits = 4096;   // types.path_edit_max_edits
-constexpr uint32_t kPeTile = 4096;       // attributes per CTA of the rewrite
+constexpr uint32_t kPeStep = 4096;       // attributes per step of the rewrite
+constexpr uint32_t kPeSteps = 4;
+constexpr uint32_t kPeTile = kPeStep * kPeSteps;  // ... and per CTA
 constexpr uint32_t kPePrimCache = 1024;  // prims of a job whose cells the walk keeps in shared memory
 constexpr uint32_t kPeBoxWarps = kWarps;  // prims per CTA of the boxes
 
@@ -404,97 +406,123 @@ __global__ void __launch_bounds__(kBlock) k_path_map(PathEditDesc p) {
     }
 }
 
-// 3. Attributes of every job, kPeTile outputs per CTA (pathedit.zig:370-425). The CTA
-// adds up the operations before its tile; a tile that none of them lies in is a copy at
-// one distance, else the distances come from a scan over the tile in shared memory.
+// 3. Attributes of every job, kPeTile outputs per CTA in kPeSteps steps (pathedit.zig:
+// 370-425). The CTA adds up the operations before each of its steps; a step that none of
+// them lies in is a copy at one distance, else the distances come from a scan over the
+// step in shared memory. Four steps per CTA share its look-ups, which are five round trips
+// before the first copy: 200 M attributes take 354 us, 656 with one step.
 __global__ void __launch_bounds__(kBlock) k_path_attrs(PathEditDesc p) {
     grid_dep_wait();
-    __shared__ int32_t s_dist[kPeTile];   // old rank - new rank
-    __shared__ uint32_t s_took[kPeTile];  // the last operation (+ 1) that took the place
+    __shared__ int32_t s_dist[kPeStep];   // old rank - new rank
+    __shared__ uint32_t s_took[kPeStep];  // the last operation (+ 1) that took the place
     __shared__ uint32_t s_scan[2 * kWarps + 2];
+    __shared__ uint32_t s_before[kWarps][kPeSteps + 1];  // per step; whether an operation lies in it
+    const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t tile = blockIdx.x;
     const uint32_t j = warp_upper_index(p.attr_tile, p.count + 1, tile);
     if (j >= p.count) return;
     const PathEditJob& job = p.jobs[j];
-    if (job.out_flags & kPeEmpty) return;
     const uint32_t n_ops = min(job.edit_count, kPeMaxEdits), n_final = job.out_count;
-    const uint32_t t0 = (tile - __ldg(p.attr_tile + j)) * kPeTile, t1 = min(t0 + kPeTile, n_final);
-    if (t0 >= n_final) return;
+    const uint32_t tile0 = (tile - __ldg(p.attr_tile + j)) * kPeTile;
+    if ((job.out_flags & kPeEmpty) || tile0 >= n_final) return;
     const uint4* ops = p.edits + job.edit_first;
-    uint32_t before = 0;  // as a difference: may wrap
-    bool inside = false;
-    for (uint32_t k = threadIdx.x; k < n_ops; k += kBlock) {
-        const uint4 o = ops[k];
-        if (o.x == kPeMapInsert) before -= o.y < t0 ? 1u : 0u;
-        if (o.x == kPeMapRemove) before += o.y <= t0 ? 1u : 0u;
-        inside |= o.x != 0 && o.y >= t0 && o.y < t1;
-    }
-    inside = __syncthreads_or(inside);
-    uint32_t dist0;
-    block_excl_scan(before, s_scan, &dist0);
-    constexpr uint32_t kPer = kPeTile / kBlock;
-    if (inside) {
-        for (uint32_t k = threadIdx.x; k < kPeTile; k += kBlock) { s_dist[k] = 0; s_took[k] = 0; }
-        __syncthreads();
+    {
+        uint32_t before[kPeSteps] = {}, inside = 0;  // (differences: may wrap)
         for (uint32_t k = threadIdx.x; k < n_ops; k += kBlock) {
             const uint4 o = ops[k];
-            if (o.x == 0 || o.y < t0 || o.y >= t1) continue;
-            const uint32_t i = o.y - t0;
-            if (o.x == kPeMapRemove) {
-                if (i > 0) atomicAdd(s_dist + i, 1);
-            } else {
-                atomicMax(s_took + i, k + 1);
-                if (o.x == kPeMapInsert && i + 1 < kPeTile) atomicAdd(s_dist + i + 1, -1);
+            if (o.x == 0) continue;
+#pragma unroll
+            for (uint32_t s = 0; s < kPeSteps; ++s) {
+                const uint32_t t0 = tile0 + s * kPeStep;
+                if (o.x == kPeMapInsert) before[s] -= o.y < t0 ? 1u : 0u;
+                if (o.x == kPeMapRemove) before[s] += o.y <= t0 ? 1u : 0u;
+                if (o.y - t0 < kPeStep) inside |= 1u << s;
             }
         }
-        __syncthreads();
-        uint32_t sum = 0, unused;
 #pragma unroll
-        for (uint32_t k = 0; k < kPer; ++k) sum += uint32_t(s_dist[threadIdx.x * kPer + k]);
-        uint32_t run = dist0 + block_excl_scan(sum, s_scan, &unused);
-#pragma unroll
-        for (uint32_t k = 0; k < kPer; ++k) {
-            run += uint32_t(s_dist[threadIdx.x * kPer + k]);
-            s_dist[threadIdx.x * kPer + k] = int32_t(run);
+        for (uint32_t s = 0; s < kPeSteps; ++s) {
+            const uint32_t sum = __reduce_add_sync(kFull, before[s]);
+            if (lane == 0) s_before[warp][s] = sum;
         }
-        __syncthreads();
+        inside = __reduce_or_sync(kFull, inside);
+        if (lane == 0) s_before[warp][kPeSteps] = inside;
     }
+    __syncthreads();
+    uint32_t in_steps = 0;
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) in_steps |= s_before[w][kPeSteps];
+    constexpr uint32_t kPer = kPeStep / kBlock;
     const uint32_t* src = p.attrs + job.attr_src;
     uint32_t* dst = p.attrs + job.attr_a;
-    if (job.palette) {
-        for (uint32_t wd = t0 / 8 + threadIdx.x; wd < (t1 + 7) / 8; wd += kBlock) {
-            const uint32_t i0 = wd * 8, n = min(t1 - i0, 8u);
-            uint32_t word = 0;
-            if (!inside) {
-                const uint32_t a = i0 + dist0, b = a + n - 1;
-                const uint32_t lo = src[a >> 3], hi = (b >> 3) != (a >> 3) ? src[b >> 3] : 0u;
-                word = __funnelshift_r(lo, hi, (a & 7) * 4);
-                if (n < 8) word &= (1u << (4 * n)) - 1;
-            } else {
-                for (uint32_t q = 0; q < n; ++q) {
-                    const uint32_t i = i0 + q - t0, took = s_took[i];
-                    const uint32_t idx = t0 + i + uint32_t(s_dist[i]);
-                    const uint32_t x = took ? ops[took - 1].z : (src[idx >> 3] >> ((idx & 7) * 4)) & 15;
-                    word |= x << (q * 4);
+    for (uint32_t s = 0; s < kPeSteps; ++s) {
+        const uint32_t t0 = tile0 + s * kPeStep, t1 = min(t0 + kPeStep, n_final);
+        if (t0 >= n_final) break;
+        const bool inside = (in_steps >> s) & 1;
+        uint32_t dist0 = 0;
+#pragma unroll
+        for (int w = 0; w < kWarps; ++w) dist0 += s_before[w][s];
+        if (inside) {
+            __syncthreads();  // the step before is done with the arrays
+            for (uint32_t k = threadIdx.x; k < kPeStep; k += kBlock) { s_dist[k] = 0; s_took[k] = 0; }
+            __syncthreads();
+            for (uint32_t k = threadIdx.x; k < n_ops; k += kBlock) {
+                const uint4 o = ops[k];
+                if (o.x == 0 || o.y - t0 >= kPeStep) continue;
+                const uint32_t i = o.y - t0;
+                if (o.x == kPeMapRemove) {
+                    if (i > 0) atomicAdd(s_dist + i, 1);
+                } else {
+                    atomicMax(s_took + i, k + 1);
+                    if (o.x == kPeMapInsert && i + 1 < kPeStep) atomicAdd(s_dist + i + 1, -1);
                 }
             }
-            dst[wd] = word;
+            __syncthreads();
+            uint32_t sum = 0, unused;
+#pragma unroll
+            for (uint32_t k = 0; k < kPer; ++k) sum += uint32_t(s_dist[threadIdx.x * kPer + k]);
+            uint32_t run = dist0 + block_excl_scan(sum, s_scan, &unused);
+#pragma unroll
+            for (uint32_t k = 0; k < kPer; ++k) {
+                run += uint32_t(s_dist[threadIdx.x * kPer + k]);
+                s_dist[threadIdx.x * kPer + k] = int32_t(run);
+            }
+            __syncthreads();
         }
-        return;
-    }
-    // (a job's target never overlaps its source)
-    uint32_t v[kPer];
+        if (job.palette) {
+            for (uint32_t wd = t0 / 8 + threadIdx.x; wd < (t1 + 7) / 8; wd += kBlock) {
+                const uint32_t i0 = wd * 8, n = min(t1 - i0, 8u);
+                uint32_t word = 0;
+                if (!inside) {
+                    const uint32_t a = i0 + dist0, b = a + n - 1;
+                    const uint32_t lo = src[a >> 3], hi = (b >> 3) != (a >> 3) ? src[b >> 3] : 0u;
+                    word = __funnelshift_r(lo, hi, (a & 7) * 4);
+                    if (n < 8) word &= (1u << (4 * n)) - 1;
+                } else {
+                    for (uint32_t q = 0; q < n; ++q) {
+                        const uint32_t i = i0 + q - t0, took = s_took[i];
+                        const uint32_t idx = t0 + i + uint32_t(s_dist[i]);
+                        const uint32_t x = took ? ops[took - 1].z : (src[idx >> 3] >> ((idx & 7) * 4)) & 15;
+                        word |= x << (q * 4);
+                    }
+                }
+                dst[wd] = word;
+            }
+            continue;
+        }
+        // (a job's target never overlaps its source)
+        uint32_t v[kPer];
 #pragma unroll
-    for (uint32_t k = 0; k < kPer; ++k) {
-        const uint32_t i = threadIdx.x + k * kBlock;
-        v[k] = 0;
-        if (t0 + i >= t1) continue;
-        const uint32_t took = inside ? s_took[i] : 0u;
-        v[k] = took ? ops[took - 1].z : src[t0 + i + (inside ? uint32_t(s_dist[i]) : dist0)];
-    }
+        for (uint32_t k = 0; k < kPer; ++k) {
+            const uint32_t i = threadIdx.x + k * kBlock;
+            v[k] = 0;
+            if (t0 + i >= t1) continue;
+            const uint32_t took = inside ? s_took[i] : 0u;
+            v[k] = took ? ops[took - 1].z : src[t0 + i + (inside ? uint32_t(s_dist[i]) : dist0)];
+        }
 #pragma unroll
-    for (uint32_t k = 0; k < kPer; ++k)
-        if (t0 + threadIdx.x + k * kBlock < t1) dst[t0 + threadIdx.x + k * kBlock] = v[k];
+        for (uint32_t k = 0; k < kPer; ++k)
+            if (t0 + threadIdx.x + k * kBlock < t1) dst[t0 + threadIdx.x + k * kBlock] = v[k];
+    }
 }
 
 // pathedit.zig:198-236: tight box of a subtree in its own coordinates
