@@ -1217,13 +1217,6 @@ __device__ __forceinline__ uint64_t node_hash(uint32_t mask, uint32_t count, con
 
 __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
-// Leaf index of brick b: its own (it owns its mask) or its mask's owner's, found
-// through the table's owner word (only bricks that repeat a mask take this gather).
-__device__ __forceinline__ uint32_t brick_ref(const BuildDesc& d, uint32_t b) {
-    const uint32_t r = __ldcg(d.bref + b);
-    return r != kNoRef ? r : __ldcg(d.bref + ~leaf_find(d, __ldcg(d.bmask + b)).z);
-}
-
 // Per-child shared arrays of the node build are padded by one slot every 8 children:
 // a thread walks its parent's children, so the lanes of a warp read children ~8 apart
 // (one parent each), which without padding hit the same banks (16-way for 8-byte
@@ -1299,13 +1292,15 @@ __device__ __forceinline__ void node_store(const LevelDesc& L, uint32_t par, con
 // of up to 7 children of the tile's last parent), heads found with warp ballots,
 // positions by a look-back scan, then every thread builds parents from shared memory.
 // Parents per thread of the node-owner kernel and children per thread of the node
-// build: large levels take 8 and 4 (tiles of 2048 parents / 1024 children), levels
+// build: large levels take 2 and 4 (tiles of 512 parents / 1024 children), levels
 // small enough to leave most SMs idle with those take 1 (tiles of 256), so that their
-// tiles spread over the whole GPU (plan_build picks per level).
+// tiles spread over the whole GPU (plan_build picks per level). Owners of 2.1 M parents
+// with 1 / 2 / 4 / 8 per thread: 166 / 155 / 166 / 170 us; of 162,000 in a level bounded by
+// 7.4 M (a 4096^3 surface): 33 / 28 / 33 / 40.
 // Small levels (NB == 1) are latency-bound: a global round trip costs about a
 // microsecond. There every load of a staging step is in flight together, and each parent
 // (at most one per thread) is assembled before the look-back.
-constexpr int kNodeIT = 8;
+constexpr int kNodeIT = 2;
 constexpr int kNodeTile = kBlock * kNodeIT;     // tile of the node-owner kernel (large levels)
 constexpr int kNBIT = 4;
 constexpr int kNodeBuildTile = kBlock * kNBIT;  // children per node-build tile (large levels)
@@ -1400,35 +1395,52 @@ __device__ __forceinline__ void node_build_tile(const BuildDesc& d, const LevelD
             }
         }
     } else {
-        // stage the children: coalesced loads; references of bricks from the dense
-        // leaf-reference array, of nodes by one gather per child from the level's table
-        // (every slot index loaded before the gathers, so that they are all in flight)
+        // stage the children, in two steps of loads that are all in flight: references of
+        // bricks from the dense leaf-reference array, of nodes by one gather per child from
+        // the level's table; then the records (16.8 M bricks: 437 us with a load at a time,
+        // now 355)
         if (L.lv == 2) {
-            for (uint32_t i = threadIdx.x; i < tn; i += kBlock) sref[cpad(i)] = brick_ref(d, t0 + i);
+            uint32_t ref[SPT], first[SPT];
+            uint64_t key[SPT], m[SPT];
+#pragma unroll
+            for (int r = 0; r < SPT; ++r) {
+                const uint32_t i = threadIdx.x + r * kBlock;
+                ref[r] = i < tn ? __ldcg(d.bref + t0 + i) : 0u;
+                m[r] = i < tn ? L.cmask[t0 + i] : 0;
+                key[r] = i < tn ? L.ckey[t0 + i] : 0;
+                first[r] = i < tn ? L.cfirst[t0 + i] : 0u;
+            }
+#pragma unroll
+            for (int r = 0; r < SPT; ++r) {
+                const uint32_t i = threadIdx.x + r * kBlock, pi = cpad(i);
+                if (i >= tn) continue;
+                // a brick that repeats a mask takes the leaf index of the mask's owner
+                sref[pi] = ref[r] != kNoRef ? ref[r] : __ldcg(d.bref + ~leaf_find(d, m[r]).z);
+                skey[pi] = key[r];
+                sfirst[pi] = first[r];
+                scnt[pi] = __popcll(m[r]);
+                if (L.need_box) slo[pi] = m[r];
+            }
         } else {
-            uint32_t cs[SPT];
+            uint32_t cs[SPT], cnt[SPT], first[SPT];
+            uint64_t key[SPT];
 #pragma unroll
             for (int r = 0; r < SPT; ++r) {
                 const uint32_t i = threadIdx.x + r * kBlock;
                 cs[r] = i < tn ? L.cslot[t0 + i] : 0u;
+                key[r] = i < tn ? L.ckey[t0 + i] : 0;
+                cnt[r] = i < tn ? L.ccnt[t0 + i] : 0u;
+                first[r] = i < tn ? L.cfirst[t0 + i] : 0u;
             }
 #pragma unroll
             for (int r = 0; r < SPT; ++r) {
-                const uint32_t i = threadIdx.x + r * kBlock;
-                if (i < tn) sref[cpad(i)] = __ldcg(&L.ctable[cs[r]].w);
-            }
-        }
-        for (uint32_t i = threadIdx.x; i < tn; i += kBlock) {
-            const uint32_t c = t0 + i, pi = cpad(i);
-            skey[pi] = L.ckey[c];
-            sfirst[pi] = L.cfirst[c];
-            if (L.lv == 2) {
-                const uint64_t m = L.cmask[c];
-                scnt[pi] = __popcll(m);
-                if (L.need_box) slo[pi] = m;
-            } else {
-                scnt[pi] = L.ccnt[c];
-                if (L.need_box) { slo[pi] = L.clo[c]; shi[pi] = L.chi[c]; }
+                const uint32_t i = threadIdx.x + r * kBlock, pi = cpad(i);
+                if (i >= tn) continue;
+                sref[pi] = __ldcg(&L.ctable[cs[r]].w);
+                skey[pi] = key[r];
+                sfirst[pi] = first[r];
+                scnt[pi] = cnt[r];
+                if (L.need_box) { slo[pi] = L.clo[t0 + i]; shi[pi] = L.chi[t0 + i]; }
             }
         }
     }
