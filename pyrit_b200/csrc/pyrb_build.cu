@@ -502,7 +502,11 @@ pyrb_result plan_build(const Job& job, const Tune* fixed, Plan& p) {
     } else {
         rb = p.key64 ? 8u : g_radix_bits.load();
         tile_keys = p.key64 ? 2048u : g_tile_keys.load();
-        if (rb == 0) auto_tuning(lb - 6, &rb, &tile_keys);
+        if (rb == 0) {
+            auto_tuning(lb - 6, &rb, &tile_keys);
+            // chunks that a 4096-entry tile (nearly) holds would leave 8192-entry ones half empty
+            if (K > 1 && nmax <= uint64_t(K) * 6144) tile_keys = 4096;
+        }
         lf = g_load_pct.load();
         path = g_path.load();
     }
