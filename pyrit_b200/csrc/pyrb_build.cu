@@ -294,17 +294,17 @@ uint32_t launch_levels(const BuildDesc& d, const std::vector<LevelDesc>& levels,
     return launches + 1;
 }
 
-TailDesc make_tail(uint32_t lv0, const uint32_t* P, const std::vector<LevelDesc>& levels, const uint4* leaf_table) {
+TailDesc make_tail(uint32_t lv0, const uint32_t* P, const std::vector<LevelDesc>& levels, bool down) {
     TailDesc T;
     std::memset(&T, 0, sizeof(T));
     T.lv0 = lv0;
+    T.down = down ? 1u : 0u;
     for (int i = 0; i < kMaxLevels + 2; ++i) T.parent_bound[i] = P[i];
     for (const LevelDesc& L : levels) {
         const int ps = (L.lv - 2) & 1;
         T.set[ps] = RecordSet{L.pkey, L.pcnt, L.pfirst, L.pslot, L.plo, L.phi, L.pwords};
         if (L.lv + 1 == lv0) T.ctable0 = L.ptable;
     }
-    if (lv0 == 2) T.ctable0 = leaf_table;
     return T;
 }
 
@@ -844,11 +844,6 @@ uint32_t launch_plan(const Plan& p, const std::vector<LevelDesc>& levels, cudaSt
         launch(k_grid_write<true>, d.grid_tiles, kBlock, 0, st, d);
         prof.mark("bucket_tile_write");
         launches += d.grid_fold ? 7 : 8;
-        if (d.chunked) {
-            launch(k_grid_chunks, std::max(std::min((p.K + kBlock - 1) / kBlock, 1024u), 1u), kBlock, 0, st, d);
-            prof.mark("grid_chunks");
-            ++launches;
-        }
     } else if (p.grid) {
         if (d.one_seg && d.n_old) {
             launch(k_grid_old, (d.n_old + 8 * kBlock - 1) / (8 * kBlock), kBlock, 0, st, d);
@@ -867,17 +862,15 @@ uint32_t launch_plan(const Plan& p, const std::vector<LevelDesc>& levels, cudaSt
         launch(k_grid_write<false>, d.grid_tiles, kBlock, 0, st, d);
         prof.mark("grid_write");
         launches += d.grid_fold ? 3 : 4;
-        if (d.chunked) {
-            launch(k_grid_chunks, std::max(std::min((p.K + kBlock - 1) / kBlock, 1024u), 1u), kBlock, 0, st, d);
-            prof.mark("grid_chunks");
-            ++launches;
-        }
     } else {
         if ((*err = launch_sort_any(p.rb, p.it, d, st, prof)) != cudaSuccess) return 0;
         launches += 3 + p.passes;
     }
     const uint32_t B = p.B;
-    if (d.leaf_regions > 1) {
+    const uint32_t lv0 = tail_level(d.log2, B, p.P);
+    if (lv0 == 2) {
+        // at most kTailMaxChildren bricks: the tail deduplicates the leaves, too
+    } else if (d.leaf_regions > 1) {
         launch(k_leaf_part, std::max(std::min((B + kBrickTile - 1) / kBrickTile, 148u * 8u), 1u), kBlock, 0, st, d);
         prof.mark("leaf_part");
         ++launches;
@@ -886,14 +879,16 @@ uint32_t launch_plan(const Plan& p, const std::vector<LevelDesc>& levels, cudaSt
     } else {
         launch(k_leaf_insert, leaf_insert_grid(d), kBlock, 0, st, d);
     }
-    prof.mark("leaf_insert");
-    launch(k_leaf_own, d.leafown_tiles, kBlock, 0, st, d);
-    prof.mark("leaf_own");
-    launches += 2;
-    const uint32_t lv0 = tail_level(d.log2, B, p.P);
-    launches += launch_levels(d, levels, lv0, make_tail(lv0, p.P, levels, d.leaf_table), st, prof);
-    if (d.mode == kModeBatch && p.min_log2 < d.log2) {
-        launch(k_batch_roots, std::max(std::min((p.K + 255) / 256, 1024u), 1u), 256, 0, st, d, d.log2);
+    if (lv0 > 2) {
+        prof.mark("leaf_insert");
+        launch(k_leaf_own, d.leafown_tiles, kBlock, 0, st, d);
+        prof.mark("leaf_own");
+        launches += 2;
+    }
+    const bool down = d.mode == kModeBatch && p.min_log2 < d.log2;
+    launches += launch_levels(d, levels, lv0, make_tail(lv0, p.P, levels, down), st, prof);
+    if (down && lv0 == d.log2) {  // no tail
+        launch(k_batch_roots, std::max(std::min((p.K + 255) / 256, 1024u), 1u), 256, 0, st, d);
         prof.mark("batch_roots");
         ++launches;
     }

@@ -454,7 +454,7 @@ __global__ void __launch_bounds__(kBlock, 5) k_grid_write(BuildDesc d) {
             seg_lo = seg_hi;
             seg_hi = __ldg(d.grid_off + seg + 1);
         }
-        // the voxels before a chunk's first cell (k_grid_chunks turns them into its first voxel)
+        // the voxels before a chunk's first cell (grid_chunk_first turns them into its first voxel)
         if (d.chunked && cell == seg_lo && lane == 0) d.chunk_vstart[seg] = vpos;
         const unsigned lo = __ballot_sync(kFull, a0[k] != 0), hi = __ballot_sync(kFull, a1[k] != 0);
         if (!(lo | hi)) continue;                       // warp-uniform
@@ -496,17 +496,6 @@ __global__ void __launch_bounds__(kBlock, 5) k_grid_write(BuildDesc d) {
         __syncthreads();
         if (threadIdx.x < d.leaf_regions && s_rcount[threadIdx.x])
             atomicAdd(d.region_count + threadIdx.x, s_rcount[threadIdx.x]);
-    }
-}
-
-// First voxel of every chunk of a chunk build (chunkFirst, gbuild.zig:237-242): the
-// voxels before its first cell, or 0xFFFFFFFF for a chunk without voxels.
-__global__ void __launch_bounds__(kBlock) k_grid_chunks(BuildDesc d) {
-    grid_dep_wait();
-    const uint32_t total = d.counters[kCtrUnique];
-    for (uint32_t c = blockIdx.x * kBlock + threadIdx.x; c < d.seg_count; c += gridDim.x * kBlock) {
-        const uint32_t v = d.chunk_vstart[c], next = c + 1 < d.seg_count ? d.chunk_vstart[c + 1] : total;
-        d.chunk_first[c] = next > v ? v : 0xFFFFFFFFu;
     }
 }
 

@@ -223,10 +223,11 @@ struct RecordSet {
 };
 
 struct TailDesc {
-    uint32_t lv0;                    // first level built by the tail (children <= kTailMaxChildren)
+    uint32_t lv0;                    // first level built by the tail (children <= kTailMaxChildren); 2: with the leaves
+    uint32_t down;                   // mixed batch: roots of chunks smaller than the batch's edge
     uint32_t parent_bound[kMaxLevels + 2];
     RecordSet set[2];                // parents of level lv live in set[(lv - 2) & 1]
-    const uint4* ctable0;            // references of lv0's children: leaf table (lv0 == 2) or level lv0-1 table
+    const uint4* ctable0;            // lv0 > 2: references of its children (level lv0 - 1's table)
 };
 
 

@@ -1014,6 +1014,18 @@ __global__ void __launch_bounds__(kBlock) k_leaf_part(BuildDesc d) {
     }
 }
 
+// First voxel of every chunk of a chunk build on the grid (chunkFirst, gbuild.zig:237-242):
+// the voxels before its first cell, or 0xFFFFFFFF for a chunk without voxels. By the
+// threads of the kernel after the write pass.
+__device__ __forceinline__ void grid_chunk_first(const BuildDesc& d, uint32_t t0, uint32_t stride) {
+    if (!d.chunked || !(d.use_grid | d.use_bucket)) return;
+    const uint32_t total = d.counters[kCtrUnique];
+    for (uint32_t c = t0; c < d.seg_count; c += stride) {
+        const uint32_t v = d.chunk_vstart[c], next = c + 1 < d.seg_count ? d.chunk_vstart[c + 1] : total;
+        d.chunk_first[c] = next > v ? v : 0xFFFFFFFFu;
+    }
+}
+
 // Leaf dedup insert in brick order, two bricks per thread per round. Equal masks of a
 // warp row are collapsed with match_any first: only the lowest brick of each group
 // touches the table.
@@ -1023,6 +1035,7 @@ __global__ void __launch_bounds__(kBlock) k_leaf_insert(BuildDesc d) {
     const uint32_t B = min(d.counters[kCtrBricks], d.brick_bound);
     const unsigned lane = threadIdx.x & 31;
     const uint32_t stride = gridDim.x * kBlock;
+    grid_chunk_first(d, blockIdx.x * kBlock + threadIdx.x, stride);
     for (uint32_t base = blockIdx.x * kBlock; base < B; base += N * stride) {
         bool v[N], w[N];
         uint64_t m[N];
@@ -1838,6 +1851,24 @@ __device__ __forceinline__ void tail_words(const uint32_t* words, uint32_t q, ui
     }
 }
 
+// Mixed batch: chunk c of edge 2^log2[c] < 2^top_log2 sits in the low corner of its
+// cell, so above its own top level it hangs below single-child nodes (child index
+// 0). Its root is found by descending from the cell's top node.
+__device__ __forceinline__ void batch_roots(const BuildDesc& d, uint32_t t0, uint32_t stride) {
+    for (uint32_t c = t0; c < d.seg_count; c += stride) {
+        uint32_t node = __ldcg(d.roots + c);
+        if (node == 0xFFFFFFFFu) continue;
+        const uint32_t l = __ldg(d.chunk_log2 + c);
+        for (uint32_t lv = d.log2; lv > l; --lv) node = __ldcg(d.nodes + node + 2);
+        d.roots[c] = node;
+    }
+}
+
+__global__ void k_batch_roots(BuildDesc d) {
+    grid_dep_wait();
+    batch_roots(d, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
+}
+
 // Prim q of the RT level: a parent's cell, box, first voxel and node; prev: the key of the
 // parent before it.
 __device__ __forceinline__ void tail_prim(const BuildDesc& d, uint32_t q, uint64_t full, uint64_t plo, uint64_t phi,
@@ -1897,6 +1928,7 @@ __global__ void __launch_bounds__(kTailThreads) k_tail(BuildDesc d, TailDesc T) 
         s_children = lv0 == 2 ? min(d.counters[kCtrBricks], d.brick_bound)
                               : min(d.counters[kCtrParents + lv0 - 1], T.parent_bound[lv0 - 1]);
     }
+    if (lv0 == 2) grid_chunk_first(d, tid, kTailThreads);  // (there is no leaf kernel before)
     __syncthreads();
     const uint32_t local_shift = 3 * (d.log2 - d.rt_log2);
     bool staged = false;  // the children are in shared memory: the parents of a small level
@@ -1910,32 +1942,57 @@ __global__ void __launch_bounds__(kTailThreads) k_tail(BuildDesc d, TailDesc T) 
         // 1. stage children (coalesced: child tid + k * kTailThreads)
         if (staged) {
         } else if (lv == 2) {
-            uint64_t key[kTailPer], mask[kTailPer];
-            uint32_t ref[kTailPer], own[kTailPer];
+            // the leaves as well: masks deduplicated in the table of the large levels (owner =
+            // minimum brick index), owners numbered in brick order
+            for (uint32_t i = tid; i < kTailSlots; i += kTailThreads) { tkey[i] = 0; towner[i] = 0xFFFFFFFFu; }
+            uint64_t mask[kTailPer];
 #pragma unroll
             for (uint32_t k = 0; k < kTailPer; ++k) {
                 const uint32_t i = tid + k * kTailThreads;
-                const bool v = i < C;
-                key[k] = v ? d.bkey[i] : 0;
-                mask[k] = v ? d.bmask[i] : 0;
-                ref[k] = v ? __ldcg(d.bref + i) : 0;
-            }
-            // a brick that repeats a mask takes the leaf index of the mask's owner
-#pragma unroll
-            for (uint32_t k = 0; k < kTailPer; ++k)
-                own[k] = ref[k] == kNoRef ? ~leaf_find(d, mask[k]).z : 0;
-#pragma unroll
-            for (uint32_t k = 0; k < kTailPer; ++k)
-                if (ref[k] == kNoRef) ref[k] = __ldcg(d.bref + own[k]);
-#pragma unroll
-            for (uint32_t k = 0; k < kTailPer; ++k) {
-                const uint32_t i = tid + k * kTailThreads;
+                mask[k] = i < C ? d.bmask[i] : 0;
                 if (i < C) {
-                    skey[i] = key[k];
+                    skey[i] = d.bkey[i];
                     slo[i] = mask[k];
-                    sref[i] = ref[k];
                     scnt[i] = __popcll(mask[k]);
                 }
+            }
+            __syncthreads();
+#pragma unroll
+            for (uint32_t k = 0; k < kTailPer; ++k) {
+                const uint32_t i = tid + k * kTailThreads;
+                if (i >= C) continue;
+                uint32_t h = uint32_t(mix64(mask[k])) & (kTailSlots - 1);
+                while (true) {  // at most half of the slots are taken
+                    const uint32_t cur = atomicCAS(tkey + h, 0u, i + 1);
+                    if (cur == 0 || slo[cur - 1] == mask[k]) break;
+                    h = (h + 1) & (kTailSlots - 1);
+                }
+                pslot[i] = uint16_t(h);
+                atomicMin(towner + h, i);
+            }
+            __syncthreads();
+            uint32_t owners = 0;
+#pragma unroll
+            for (uint32_t k = 0; k < kTailPer; ++k) {
+                const uint32_t i = tid * kTailPer + k;
+                owners += i < C && towner[pslot[i]] == i ? 1u : 0u;
+            }
+            uint32_t total;
+            uint32_t pos = tail_scan1(owners, scan + 32, &total);
+#pragma unroll
+            for (uint32_t k = 0; k < kTailPer; ++k) {
+                const uint32_t i = tid * kTailPer + k;
+                if (i < C && towner[pslot[i]] == i) {
+                    d.leaves[pos] = slo[i];
+                    pval[i] = pos++;
+                }
+            }
+            if (tid == 0) d.counters[kCtrLeaves] = total;
+            __syncthreads();
+#pragma unroll
+            for (uint32_t k = 0; k < kTailPer; ++k) {
+                const uint32_t i = tid + k * kTailThreads;
+                if (i < C) sref[i] = pval[towner[pslot[i]]];
             }
         } else {
             uint64_t key[kTailPer], lo[kTailPer], hi[kTailPer];
@@ -2239,6 +2296,7 @@ __global__ void __launch_bounds__(kTailThreads) k_tail(BuildDesc d, TailDesc T) 
         }
         __syncthreads();
     }
+    if (T.down) batch_roots(d, tid, kTailThreads);  // (every level ended with a barrier)
     if (tid == 0) {
         // final counts and the empty geometry (gbuild.zig:607-624)
         const uint32_t top_set = (d.log2 - 1 - 2) & 1;
@@ -2255,20 +2313,6 @@ __global__ void __launch_bounds__(kTailThreads) k_tail(BuildDesc d, TailDesc T) 
         }
         d.counters[kCtrRoot] = root;
         d.counters[kCtrWords] = cursor;
-    }
-}
-
-// Mixed batch: chunk c of edge 2^log2[c] < 2^top_log2 sits in the low corner of its
-// cell, so above its own top level it hangs below single-child nodes (child index
-// 0). Its root is found by descending from the cell's top node.
-__global__ void k_batch_roots(BuildDesc d, uint32_t max_log2) {
-    grid_dep_wait();
-    for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < d.seg_count; c += gridDim.x * blockDim.x) {
-        uint32_t node = d.roots[c];
-        if (node == 0xFFFFFFFFu) continue;
-        const uint32_t l = __ldg(d.chunk_log2 + c);
-        for (uint32_t lv = max_log2; lv > l; --lv) node = d.nodes[node + 2];
-        d.roots[c] = node;
     }
 }
 
