@@ -589,8 +589,9 @@ pyrb_result plan_build(const Job& job, const Tune* fixed, Plan& p) {
     d.leaf_regions = 1;
     while (K == 1 && d.leaf_regions < kMaxLeafRegions && d.leaf_cap / d.leaf_regions > kLeafRegionSlots)
         d.leaf_regions <<= 1;
-    d.leaf_region_shift = 0;
-    while ((d.leaf_cap >> d.leaf_region_shift) > d.leaf_regions) ++d.leaf_region_shift;
+    d.leaf_region_shift = 32;
+    while ((1u << (32 - d.leaf_region_shift)) < d.leaf_regions) --d.leaf_region_shift;
+    d.load_pct = lf;
     d.node_bound = uint32_t(words);
     d.prim_bound = P[rt - 1];
     if (p.grid || p.bucket) {
@@ -626,7 +627,6 @@ pyrb_result plan_build(const Job& job, const Tune* fixed, Plan& p) {
         p.oit[lv] = P[lv] >= kSmallLevelTiles * kNodeTile ? kNodeIT : 1;
         p.btiles[lv] = std::max((child + kBlock * p.bnb[lv] - 1) / (kBlock * p.bnb[lv]), 1u);
         p.otiles[lv] = std::max((P[lv] + kBlock * p.oit[lv] - 1) / (kBlock * p.oit[lv]), 1u);
-        p.o_table[lv] = zl.take(uint64_t(p.cap[lv]) * 16);
         p.o_bstat[lv] = zl.take(uint64_t(p.btiles[lv]) * 8);
         p.o_ostat[lv] = zl.take(uint64_t(p.otiles[lv]) * 8);
     }
@@ -643,6 +643,8 @@ pyrb_result plan_build(const Job& job, const Tune* fixed, Plan& p) {
     Layout ol;
     ol.size = p.zero_bytes + p.ff_bytes;
     if (d.leaf_regions > 1) p.o_leaf_table = ol.take(uint64_t(d.leaf_cap) * 16);
+    // (cleared by the level's build kernel, as far as its real children need)
+    for (uint32_t lv = 2; lv < log2; ++lv) p.o_table[lv] = ol.take(uint64_t(p.cap[lv]) * 16);
     p.o_seg_entry = ol.take(uint64_t(K + 1) * 4);
     p.o_seg_tile = ol.take(uint64_t(K + 1) * 4);
     const uint64_t kbytes = p.key64 ? 8 : 4;
@@ -816,7 +818,7 @@ uint32_t launch_plan(const Plan& p, const std::vector<LevelDesc>& levels, cudaSt
     Prof prof(st);
     uint8_t* base = reinterpret_cast<uint8_t*>(d.counters) - p.o_counters;
     *err = cudaMemsetAsync(base, 0, p.zero_bytes, st);
-    if (*err == cudaSuccess) *err = cudaMemsetAsync(base + p.zero_bytes, 0xFF, p.ff_bytes, st);
+    if (*err == cudaSuccess && p.chunked) *err = cudaMemsetAsync(base + p.zero_bytes, 0xFF, p.ff_bytes, st);
     if (*err != cudaSuccess) return 0;
     prof.mark("memset");
     uint32_t launches = 0;

@@ -113,12 +113,13 @@ struct BuildDesc {
     uint8_t* binst;          // [B] 1: the brick made itself its mask's owner (zeroed)
     uint8_t* bdisp;          // [B] 1: ... and was replaced by a smaller brick index (zeroed)
     uint4* leaf_table;       // {mask lo, mask hi, ~owner, leaf index}
-    uint32_t leaf_cap;
+    uint32_t leaf_cap;       // slots allocated (for brick_bound bricks; leaf_table_of: those in use)
+    uint32_t load_pct;       // load factor of the dedup tables
     // Tables larger than L2 are filled region by region: leaf_regions > 1 groups the
     // bricks by the table region (leaf_cap / leaf_regions slots) of their mask's home
     // slot first, so the inserts in flight at any time touch a slice that stays in L2.
     uint32_t leaf_regions;
-    uint32_t leaf_region_shift;  // log2(leaf_cap / leaf_regions)
+    uint32_t leaf_region_shift;  // 32 - log2(leaf_regions): the region in a hash's top bits
     uint32_t* region_count;      // [leaf_regions] bricks per region (zero-initialised)
     uint32_t* region_cursor;     // [leaf_regions] (zero-initialised)
     uint32_t* region_zeroed;     // [leaf_regions] clearing tiles finished (zero-initialised)
@@ -175,7 +176,7 @@ struct LevelDesc {
     uint32_t build_tiles;
     uint32_t own_tiles;
     uint32_t need_box;       // parents need a bounding box (lv + 1 <= rt_log2)
-    uint32_t pcap;           // table capacity (power of two)
+    uint32_t pcap;           // table slots allocated (power of two; table_slots: those in use)
     uint32_t tile_ctr_build; // counter index of the dynamic tile ids
     uint32_t tile_ctr_own;
     uint32_t build_nb;       // children per thread of the build kernel (4, or 1 for small levels)

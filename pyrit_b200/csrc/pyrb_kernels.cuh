@@ -529,9 +529,28 @@ __global__ void __launch_bounds__(NT, PYRB_SORT_MIN_BLOCKS * kBlock / NT) k_sort
 // the first sighting of a cell is its last entry, the cell's winner.
 // ---------------------------------------------------------------------------
 
+// Slots of a dedup table for `count` items: what the load factor asks for, at most the
+// allocated `bound` (sized by the largest count that the input could have).
+__device__ __forceinline__ uint32_t table_slots(const BuildDesc& d, uint32_t count, uint32_t bound) {
+    const uint64_t need = (uint64_t(count) * 100 + d.load_pct - 1) / d.load_pct;
+    if (need >= bound) return bound;
+    return need <= 1024 ? min(1024u, bound) : min(1u << (32 - __clz(uint32_t(need) - 1)), bound);
+}
+
+// The leaf table of B bricks: `slots` of them in use, a mask's home slot in the top bits of
+// its hash (so that its region is the same however many slots are used).
+struct LeafTable { uint32_t slots, shift; };
+__device__ __forceinline__ LeafTable leaf_table_of(const BuildDesc& d, uint32_t bricks) {
+    LeafTable t;
+    // (a region keeps at least 4096 slots: its share of the masks varies)
+    t.slots = min(max(table_slots(d, bricks, d.leaf_cap), d.leaf_regions > 1 ? d.leaf_regions * 4096 : 1u), d.leaf_cap);
+    t.shift = 32 - (31 - __clz(t.slots));
+    return t;
+}
+__device__ __forceinline__ uint32_t leaf_home(const LeafTable& t, uint64_t mask) { return uint32_t(mix64(mask)) >> t.shift; }
 // Table region of a mask's home slot (see BuildDesc::leaf_regions).
 __device__ __forceinline__ uint32_t leaf_region(const BuildDesc& d, uint64_t mask) {
-    return (uint32_t(mix64(mask)) & (d.leaf_cap - 1)) >> d.leaf_region_shift;
+    return uint32_t(mix64(mask)) >> d.leaf_region_shift;
 }
 
 template <int IT, typename KeyT>
@@ -890,7 +909,7 @@ __device__ __forceinline__ uint32_t leaf_insert_at(const BuildDesc& d, uint4* ta
 // takes N bricks per round: the inserts are latency-bound on random table slots).
 // out[k]: slot | kInstalled.
 template <int N>
-__device__ __forceinline__ void leaf_insert_n(const BuildDesc& d, uint4* table, uint32_t cap, uint32_t smask,
+__device__ __forceinline__ void leaf_insert_n(const BuildDesc& d, uint4* table, const LeafTable& t, uint32_t smask,
                                               const bool (&w)[N], const uint64_t (&m)[N], const uint32_t (&idx)[N],
                                               uint32_t (&out)[N]) {
     uint32_t h[N], z[N];
@@ -898,7 +917,7 @@ __device__ __forceinline__ void leaf_insert_n(const BuildDesc& d, uint4* table, 
     bool f[N];
 #pragma unroll
     for (int k = 0; k < N; ++k) {
-        h[k] = uint32_t(mix64(m[k])) & (cap - 1);
+        h[k] = leaf_home(t, m[k]);
         // the slot's first 16 bytes as one load: mask and (possibly older) ~owner
         const uint4 c = w[k] ? __ldcg(table + h[k]) : make_uint4(0, 0, 0, 0);
         r[k] = uint64_t(c.y) << 32 | c.x;
@@ -925,9 +944,9 @@ __device__ __forceinline__ void leaf_insert_n(const BuildDesc& d, uint4* table, 
 
 // The slot holding `mask` (it was inserted): the same probe sequence as the insert,
 // each probe one 16-byte load that also returns the slot's ~owner.
-__device__ __forceinline__ uint4 leaf_find(const BuildDesc& d, uint64_t mask) {
-    const uint32_t smask = d.leaf_regions > 1 ? d.leaf_cap / d.leaf_regions - 1 : d.leaf_cap - 1;
-    uint32_t h = uint32_t(mix64(mask)) & (d.leaf_cap - 1);
+__device__ __forceinline__ uint4 leaf_find(const BuildDesc& d, const LeafTable& t, uint64_t mask) {
+    const uint32_t smask = (d.leaf_regions > 1 ? t.slots / d.leaf_regions : t.slots) - 1;
+    uint32_t h = leaf_home(t, mask);
     for (uint32_t probe = 0; probe <= smask; ++probe) {
         const uint4 v = __ldcg(d.leaf_table + h);
         if ((uint64_t(v.y) << 32 | v.x) == mask) return v;
@@ -1036,6 +1055,7 @@ __global__ void __launch_bounds__(kBlock) k_leaf_insert(BuildDesc d) {
     const unsigned lane = threadIdx.x & 31;
     const uint32_t stride = gridDim.x * kBlock;
     grid_chunk_first(d, blockIdx.x * kBlock + threadIdx.x, stride);
+    const LeafTable t = leaf_table_of(d, B);
     for (uint32_t base = blockIdx.x * kBlock; base < B; base += N * stride) {
         bool v[N], w[N];
         uint64_t m[N];
@@ -1052,7 +1072,7 @@ __global__ void __launch_bounds__(kBlock) k_leaf_insert(BuildDesc d) {
             w[k] = v[k] && lane == l[k];
             s[k] = 0;
         }
-        leaf_insert_n<N>(d, d.leaf_table, d.leaf_cap, d.leaf_cap - 1, w, m, b, s);
+        leaf_insert_n<N>(d, d.leaf_table, t, t.slots - 1, w, m, b, s);
 #pragma unroll
         for (int k = 0; k < N; ++k) {
             s[k] = __shfl_sync(kFull, s[k], l[k]);
@@ -1091,7 +1111,9 @@ __global__ void __launch_bounds__(kBlock) k_leaf_insert_regions(BuildDesc d) {
     grid_dep_wait();
     __shared__ uint32_t s_tile;
     __shared__ uint32_t s_tbase[kMaxLeafRegions + 1], s_ibase[kMaxLeafRegions + 1];
-    const uint32_t R = d.leaf_regions, S = d.leaf_cap / R, smask = S - 1;
+    const uint32_t B = min(d.counters[kCtrBricks], d.brick_bound);
+    const LeafTable t = leaf_table_of(d, B);
+    const uint32_t R = d.leaf_regions, S = t.slots / R, smask = S - 1;
     const uint32_t nz = (S + kZeroSlots - 1) / kZeroSlots;
     if (threadIdx.x < 32) region_bases(d, nz, kInsTile, s_tbase, s_ibase);
     const uint32_t tile = dyn_tile(d.counters, kTileLeafInsert, &s_tile);  // its barrier publishes s_tbase
@@ -1118,7 +1140,6 @@ __global__ void __launch_bounds__(kBlock) k_leaf_insert_regions(BuildDesc d) {
         }
     }
     __syncthreads();
-    const uint32_t B = min(d.counters[kCtrBricks], d.brick_bound);
     const unsigned lane = threadIdx.x & 31;
     constexpr int N = kInsPerThread;
     const uint32_t iend = s_ibase[r + 1];
@@ -1140,7 +1161,7 @@ __global__ void __launch_bounds__(kBlock) k_leaf_insert_regions(BuildDesc d) {
         w[q] = v[q] && lane == l[q];
         s[q] = 0;
     }
-    leaf_insert_n<N>(d, d.leaf_table, d.leaf_cap, smask, w, m, b, s);
+    leaf_insert_n<N>(d, d.leaf_table, t, smask, w, m, b, s);
 #pragma unroll
     for (int q = 0; q < N; ++q) {
         s[q] = __shfl_sync(kFull, s[q], l[q]);
@@ -1227,8 +1248,6 @@ __device__ __forceinline__ uint64_t node_hash(uint32_t mask, uint32_t count, con
         if (k < n) h = mix64(h ^ refs[k]);
     return h;
 }
-
-__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
 // Per-child shared arrays of the node build are padded by one slot every 8 children:
 // a thread walks its parent's children, so the lanes of a warp read children ~8 apart
@@ -1347,6 +1366,11 @@ __device__ __forceinline__ void node_build_tile(const BuildDesc& d, const LevelD
     const uint32_t C = min(children, L.lv == 2 ? d.brick_bound : L.child_bound);
     const uint32_t ntiles = (C + kTile - 1) / kTile;
     if (tile >= ntiles) return;
+    // the level's table for the inserts that follow: every tile clears its share
+    const uint32_t slots = table_slots(d, C, L.pcap);
+    for (uint32_t s = uint64_t(slots) * tile / ntiles + threadIdx.x; s < uint64_t(slots) * (tile + 1) / ntiles; s += kBlock)
+        L.ptable[s] = make_uint4(0u, 0u, 0u, 0u);
+    const LeafTable leaves = L.lv == 2 ? leaf_table_of(d, C) : LeafTable{1, 31};
     const uint32_t t0 = tile * kTile;
     const uint32_t own_n = min(uint32_t(kTile), C - t0);
     const uint32_t tn = min(uint32_t(N), C - t0);
@@ -1383,7 +1407,7 @@ __device__ __forceinline__ void node_build_tile(const BuildDesc& d, const LevelD
             uint32_t own[SPT];
 #pragma unroll
             for (int r = 0; r < SPT; ++r)
-                own[r] = threadIdx.x + r * kBlock < tn && ref[r] == kNoRef ? ~leaf_find(d, lo[r]).z : 0;
+                own[r] = threadIdx.x + r * kBlock < tn && ref[r] == kNoRef ? ~leaf_find(d, leaves, lo[r]).z : 0;
 #pragma unroll
             for (int r = 0; r < SPT; ++r)
                 if (threadIdx.x + r * kBlock < tn && ref[r] == kNoRef) ref[r] = __ldcg(d.bref + own[r]);
@@ -1428,7 +1452,7 @@ __device__ __forceinline__ void node_build_tile(const BuildDesc& d, const LevelD
                 const uint32_t i = threadIdx.x + r * kBlock, pi = cpad(i);
                 if (i >= tn) continue;
                 // a brick that repeats a mask takes the leaf index of the mask's owner
-                sref[pi] = ref[r] != kNoRef ? ref[r] : __ldcg(d.bref + ~leaf_find(d, m[r]).z);
+                sref[pi] = ref[r] != kNoRef ? ref[r] : __ldcg(d.bref + ~leaf_find(d, leaves, m[r]).z);
                 skey[pi] = key[r];
                 sfirst[pi] = first[r];
                 scnt[pi] = __popcll(m[r]);
@@ -1494,7 +1518,6 @@ __device__ __forceinline__ void node_build_tile(const BuildDesc& d, const LevelD
             return;
         }
         const uint32_t hash = uint32_t(node_hash(q.mask, q.count, q.refs, q.n));
-        prefetch_l2(&L.ptable[hash & (L.pcap - 1)]);
         node_store(L, par, q, skey[cpad(i)] >> 3, sfirst[cpad(i)], hash);
     };
     NodeParent q;
@@ -1543,7 +1566,10 @@ __global__ void __launch_bounds__(kBlock, NB == 1 ? 6 : 5) k_node_build(BuildDes
 constexpr int kProbes = 4;
 __global__ void __launch_bounds__(kBlock) k_node_insert(BuildDesc d, LevelDesc L) {
     grid_dep_wait();
-    const uint32_t P = min(__ldcg(d.counters + kCtrParents + L.lv), L.parent_bound), cmask = L.pcap - 1;
+    const uint32_t P = min(__ldcg(d.counters + kCtrParents + L.lv), L.parent_bound);
+    const uint32_t C = L.lv == 2 ? min(__ldcg(d.counters + kCtrBricks), d.brick_bound)
+                                 : min(__ldcg(d.counters + kCtrParents + L.lv - 1), L.child_bound);
+    const uint32_t cmask = table_slots(d, C, L.pcap) - 1;  // (those that the build kernel cleared)
     for (uint32_t par = blockIdx.x * kBlock + threadIdx.x; par < P; par += gridDim.x * kBlock) {
         const uint32_t hash = __ldcg(L.pslot + par);
         uint32_t h = hash & cmask, w[kNodeStride];
