@@ -12,6 +12,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <initializer_list>
 #include <mutex>
 #include <vector>
 
@@ -1337,14 +1338,21 @@ PYRB_API pyrb_result pyrb_pyrd_load(const pyrb_exec* e, const void* data, uint64
 // Chunk attribute palettes (src/device/palette.zig, src/context.zig:1311-1360)
 // ---------------------------------------------------------------------------
 namespace {
-// Device copies of the per-chunk host arrays plus the tile plan; freed stream-ordered.
+// The per-chunk host arrays and the tile plan in one device block with the call's work
+// space behind them; freed stream-ordered.
 struct PaletteJob {
     Mem mem;
     PaletteDesc p = {};
-    uint64_t blocks[4] = {};
+    uint64_t block = 0;
     uint32_t tiles = 0;
-    pyrb_result setup(const uint32_t* first, uint32_t count) {
-        std::vector<uint32_t> tile_of(count + 1);
+    std::vector<uint32_t> host;  // first, tile_of, then `more` arrays of `count`
+    // more: further host arrays of count values to upload; work: bytes behind them (8-byte
+    // aligned). *arrays and *space: their device addresses.
+    pyrb_result setup(const uint32_t* first, uint32_t count, std::initializer_list<const uint32_t*> more, uint64_t work,
+                      uint32_t** arrays, uint32_t** space) {
+        host.resize(2 * (uint64_t(count) + 1) + more.size() * uint64_t(count));
+        std::memcpy(host.data(), first, uint64_t(count + 1) * 4);
+        uint32_t* tile_of = host.data() + count + 1;
         uint64_t t = 0;
         for (uint32_t c = 0; c < count; ++c) {
             if (first[c + 1] < first[c]) return fail(PYRB_ERROR_INVALID_ARGUMENT, "first[%u] > first[%u]", c, c + 1);
@@ -1355,25 +1363,24 @@ struct PaletteJob {
         }
         tile_of[count] = uint32_t(t);
         tiles = uint32_t(t);
-        blocks[0] = mem.get(uint64_t(count + 1) * 8);
-        if (!blocks[0]) return fail(PYRB_ERROR_OUT_OF_MEMORY, "device memory for the palette plan");
-        uint32_t* dfirst = reinterpret_cast<uint32_t*>(blocks[0]);
-        CU(cudaMemcpyAsync(dfirst, first, uint64_t(count + 1) * 4, cudaMemcpyHostToDevice, mem.st));
-        CU(cudaMemcpyAsync(dfirst + count + 1, tile_of.data(), uint64_t(count + 1) * 4, cudaMemcpyHostToDevice,
-                           mem.st));
-        CU(cudaStreamSynchronize(mem.st));  // the host vector goes out of scope
-        p.first = dfirst;
-        p.tile_of = dfirst + count + 1;
+        uint32_t* to = tile_of + count + 1;
+        for (const uint32_t* m : more) {
+            std::memcpy(to, m, uint64_t(count) * 4);
+            to += count;
+        }
+        const uint64_t bytes = align_up(host.size() * 4, 256);
+        block = mem.get(bytes + work);
+        if (!block) return fail(PYRB_ERROR_OUT_OF_MEMORY, "device memory for the palettes");
+        // (the host copy lives until the call's own synchronisation)
+        CU(cudaMemcpyAsync(reinterpret_cast<void*>(block), host.data(), host.size() * 4, cudaMemcpyHostToDevice, mem.st));
+        p.first = reinterpret_cast<uint32_t*>(block);
+        p.tile_of = p.first + count + 1;
         p.count = count;
+        *arrays = reinterpret_cast<uint32_t*>(block) + 2 * (uint64_t(count) + 1);
+        *space = reinterpret_cast<uint32_t*>(block + bytes);
         return PYRB_OK;
     }
-    uint32_t* take(int k, uint64_t bytes) {
-        blocks[k] = mem.get(bytes);
-        return reinterpret_cast<uint32_t*>(blocks[k]);
-    }
-    ~PaletteJob() {
-        for (uint64_t b : blocks) mem.put(b);
-    }
+    ~PaletteJob() { mem.put(block); }
 };
 }  // namespace
 
@@ -1383,13 +1390,12 @@ PYRB_API pyrb_result pyrb_palette_scan(const pyrb_exec* e, uint64_t attrs, const
     if (count == 0) return PYRB_OK;
     if (first[count] > first[0] && !attrs) return fail(PYRB_ERROR_INVALID_ARGUMENT, "attrs is NULL");
     PaletteJob j{Mem{e, e ? reinterpret_cast<cudaStream_t>(e->stream) : nullptr}};
-    pyrb_result r = j.setup(first, count);
+    uint32_t *unused, *tab;
+    const pyrb_result r = j.setup(first, count, {}, uint64_t(count) * (kPalSlots * 8 + 8), &unused, &tab);
     if (r != PYRB_OK) return r;
     const cudaStream_t st = j.mem.st;
     j.p.attrs = reinterpret_cast<const uint32_t*>(attrs);
-    uint32_t* tab = j.take(1, uint64_t(count) * kPalSlots * 8);
-    uint32_t* small = j.take(2, uint64_t(count) * 8);
-    if (!tab || !small) return fail(PYRB_ERROR_OUT_OF_MEMORY, "device memory for the palette tables");
+    uint32_t* small = tab + uint64_t(count) * kPalSlots * 2;
     j.p.gval = tab;
     j.p.gfirst = tab + uint64_t(count) * kPalSlots;
     j.p.gflag = small;
@@ -1412,13 +1418,10 @@ PYRB_API pyrb_result pyrb_palette_pack(const pyrb_exec* e, uint64_t attrs, const
     if (count == 0) return PYRB_OK;
     if (first[count] > first[0] && !attrs) return fail(PYRB_ERROR_INVALID_ARGUMENT, "attrs is NULL");
     PaletteJob j{Mem{e, e ? reinterpret_cast<cudaStream_t>(e->stream) : nullptr}};
-    pyrb_result r = j.setup(first, count);
+    uint32_t *small, *unused;
+    const pyrb_result r = j.setup(first, count, {counts, dst}, 16, &small, &unused);
     if (r != PYRB_OK) return r;
     const cudaStream_t st = j.mem.st;
-    uint32_t* small = j.take(1, uint64_t(count) * 8);
-    if (!small) return fail(PYRB_ERROR_OUT_OF_MEMORY, "device memory for the palette plan");
-    CU(cudaMemcpyAsync(small, counts, uint64_t(count) * 4, cudaMemcpyHostToDevice, st));
-    CU(cudaMemcpyAsync(small + count, dst, uint64_t(count) * 4, cudaMemcpyHostToDevice, st));
     j.p.attrs = reinterpret_cast<const uint32_t*>(attrs);
     j.p.palettes = reinterpret_cast<uint32_t*>(palettes);
     j.p.counts = small;
@@ -1443,7 +1446,12 @@ PYRB_API pyrb_result pyrb_path_edit(const pyrb_exec* e, uint64_t nodes, uint64_t
     if (!jobs || !nodes || !leaves || !attributes || (n_edits && !edits))
         return fail(PYRB_ERROR_INVALID_ARGUMENT, "NULL pointer");
     uint32_t max_edits = 1;
-    std::vector<uint32_t> attr_tile(count + 1), prim_tile(count + 1);
+    // the jobs and their tiles in one block, one upload
+    const uint64_t jobs_bytes = align_up(uint64_t(count) * sizeof(PathEditJob), 256);
+    std::vector<uint8_t> plan(jobs_bytes + uint64_t(count + 1) * 8);
+    std::memcpy(plan.data(), jobs, uint64_t(count) * sizeof(PathEditJob));
+    uint32_t* attr_tile = reinterpret_cast<uint32_t*>(plan.data() + jobs_bytes);
+    uint32_t* prim_tile = attr_tile + count + 1;
     uint64_t at = 0, pt = 0;
     for (uint32_t j = 0; j < count; ++j) {
         const pyrb_path_edit_job& jb = jobs[j];
@@ -1466,50 +1474,32 @@ PYRB_API pyrb_result pyrb_path_edit(const pyrb_exec* e, uint64_t nodes, uint64_t
     attr_tile[count] = uint32_t(at);
     prim_tile[count] = uint32_t(pt);
     if (at >= (uint64_t(1) << 31) || pt >= (uint64_t(1) << 31)) return fail(PYRB_ERROR_INVALID_ARGUMENT, "too many attributes");
-    // Context.pathEdit: each job's edits stably ordered by brick, so that a brick is
-    // one run (one new path per brick rather than per voxel)
-    std::vector<uint32_t> sorted(uint64_t(std::max(n_edits, 1u)) * 4, 0);
-    if (n_edits) std::memcpy(sorted.data(), edits, uint64_t(n_edits) * 16);
-    for (uint32_t j = 0; j < count; ++j) {
-        std::vector<std::array<uint32_t, 4>> v(jobs[j].edit_count);
-        for (uint32_t k = 0; k < jobs[j].edit_count; ++k)
-            std::memcpy(v[k].data(), edits + uint64_t(jobs[j].edit_first + k) * 4, 16);
-        auto key = [](const std::array<uint32_t, 4>& a) {
-            return (uint64_t(a[2] >> 2) << 42) | (uint64_t(a[1] >> 2) << 21) | uint64_t(a[0] >> 2);
-        };
-        std::stable_sort(v.begin(), v.end(), [&](const std::array<uint32_t, 4>& a, const std::array<uint32_t, 4>& b) {
-            return key(a) < key(b);
-        });
-        for (uint32_t k = 0; k < jobs[j].edit_count; ++k)
-            std::memcpy(sorted.data() + uint64_t(jobs[j].edit_first + k) * 4, v[k].data(), 16);
-    }
     cudaStream_t st = e ? reinterpret_cast<cudaStream_t>(e->stream) : nullptr;
     Mem mem{e, st};
-    const uint64_t jobs_bytes = uint64_t(count) * sizeof(PathEditJob);
-    const uint64_t edit_bytes = uint64_t(std::max(n_edits, 1u)) * 16;
-    const uint64_t plan_bytes = uint64_t(count + 1) * 8;
-    const uint64_t block = mem.get(align_up(jobs_bytes, 256) + align_up(edit_bytes, 256) + plan_bytes);
+    const uint64_t edit_bytes = align_up(uint64_t(std::max(n_edits, 1u)) * 16, 256);
+    const uint64_t block = mem.get(align_up(plan.size(), 256) + 2 * edit_bytes);
     if (!block) return fail(PYRB_ERROR_OUT_OF_MEMORY, "device memory for the path edits");
     PathEditDesc p;
     p.nodes = reinterpret_cast<uint32_t*>(nodes);
     p.leaves = reinterpret_cast<uint64_t*>(leaves);
     p.attrs = reinterpret_cast<uint32_t*>(attributes);
     p.jobs = reinterpret_cast<PathEditJob*>(block);
-    p.edits = reinterpret_cast<uint4*>(block + align_up(jobs_bytes, 256));
-    uint32_t* plan = reinterpret_cast<uint32_t*>(block + align_up(jobs_bytes, 256) + align_up(edit_bytes, 256));
-    p.attr_tile = plan;
-    p.prim_tile = plan + count + 1;
+    p.attr_tile = reinterpret_cast<uint32_t*>(block + jobs_bytes);
+    p.prim_tile = p.attr_tile + count + 1;
+    uint4* given = reinterpret_cast<uint4*>(block + align_up(plan.size(), 256));
+    p.given = given;
+    p.edits = reinterpret_cast<uint4*>(reinterpret_cast<uint64_t>(given) + edit_bytes);
     p.count = count;
     auto done = [&](pyrb_result r) {
+        if (r != PYRB_OK) cudaStreamSynchronize(st);  // the caller's arrays may still be read
         mem.put(block);
         return r;
     };
-    cudaError_t err = cudaMemcpyAsync(p.jobs, jobs, jobs_bytes, cudaMemcpyHostToDevice, st);
-    if (err == cudaSuccess) err = cudaMemcpyAsync(p.edits, sorted.data(), edit_bytes, cudaMemcpyHostToDevice, st);
-    if (err == cudaSuccess) err = cudaMemcpyAsync(plan, attr_tile.data(), uint64_t(count + 1) * 4, cudaMemcpyHostToDevice, st);
-    if (err == cudaSuccess)
-        err = cudaMemcpyAsync(plan + count + 1, prim_tile.data(), uint64_t(count + 1) * 4, cudaMemcpyHostToDevice, st);
+    cudaError_t err = cudaMemcpyAsync(p.jobs, plan.data(), plan.size(), cudaMemcpyHostToDevice, st);
+    if (err == cudaSuccess && n_edits)
+        err = cudaMemcpyAsync(given, edits, uint64_t(n_edits) * 16, cudaMemcpyHostToDevice, st);
     if (err != cudaSuccess) return done(fail(PYRB_ERROR_CUDA, "path edit upload: %s", cudaGetErrorString(err)));
+    launch(k_path_sort, count, kBlock, size_t(max_edits) * sizeof(uint64_t), st, p);
     launch(k_path_walk, count, 32, 0, st, p);
     if (at) {
         launch(k_path_map, count, kBlock, size_t(max_edits) * sizeof(uint2), st, p);
@@ -1517,7 +1507,7 @@ PYRB_API pyrb_result pyrb_path_edit(const pyrb_exec* e, uint64_t nodes, uint64_t
     }
     if (pt) launch(k_path_boxes, uint32_t(pt), kBlock, 0, st, p);
     err = cudaGetLastError();
-    if (err == cudaSuccess) err = cudaMemcpyAsync(jobs, p.jobs, jobs_bytes, cudaMemcpyDeviceToHost, st);
+    if (err == cudaSuccess) err = cudaMemcpyAsync(jobs, p.jobs, uint64_t(count) * sizeof(PathEditJob), cudaMemcpyDeviceToHost, st);
     if (err == cudaSuccess) err = cudaStreamSynchronize(st);
     if (err != cudaSuccess) return done(fail(PYRB_ERROR_CUDA, "path edit: %s", cudaGetErrorString(err)));
     return done(PYRB_OK);

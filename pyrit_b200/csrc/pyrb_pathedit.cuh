@@ -59,7 +59,8 @@ struct PathEditDesc {
     uint64_t* leaves;
     uint32_t* attrs;
     PathEditJob* jobs;
-    uint4* edits;                // x, y, z, attribute; the walk makes them (op, rank, value, 0), the
+    const uint4* given;          // x, y, z, attribute, as the caller gave them
+    uint4* edits;                // the same by brick (k_path_sort); the walk makes them (op, rank, value, 0), the
                                  // attribute map (what, place, value, 0)
     const uint32_t* attr_tile;   // [count + 1] first attribute tile of each job
     const uint32_t* prim_tile;   // [count + 1] first prim tile of each job
@@ -235,6 +236,30 @@ __device__ __forceinline__ PeWalker pe_walker(const PathEditDesc& p, const PathE
     w.leaf_end = job.leaf_arena - job.leaf_offset + job.leaf_cap;
     w.overflow = false;
     return w;
+}
+
+// 0. Each job's edits stably ordered by brick, so that a brick is one run and gets one new
+// path (Context.pathEdit's sort on the host). One CTA per job: an edit's place is the
+// number of edits before it, counted over the keys in shared memory (32 edits take a few
+// us, the 4096 a job may have 0.2 ms; 256 sorts of 32 took the host 0.15 ms).
+__global__ void __launch_bounds__(kBlock) k_path_sort(PathEditDesc p) {
+    grid_dep_wait();
+    extern __shared__ uint64_t s_brick[];  // [largest edit_count of the jobs]
+    const PathEditJob& job = p.jobs[blockIdx.x];
+    const uint32_t n = min(job.edit_count, kPeMaxEdits);
+    const uint4* in = p.given + job.edit_first;
+    uint4* out = p.edits + job.edit_first;
+    for (uint32_t k = threadIdx.x; k < n; k += kBlock) {
+        const uint4 e = in[k];
+        s_brick[k] = uint64_t(e.z >> 2) << 42 | uint64_t(e.y >> 2) << 21 | uint64_t(e.x >> 2);
+    }
+    __syncthreads();
+    for (uint32_t k = threadIdx.x; k < n; k += kBlock) {
+        const uint64_t me = s_brick[k];
+        uint32_t place = 0;
+        for (uint32_t q = 0; q < n; ++q) place += s_brick[q] < me || (s_brick[q] == me && q < k) ? 1u : 0u;
+        out[place] = in[k];
+    }
 }
 
 // 1. One warp per job walks the job's bricks in order (pathedit.zig:283-368).
