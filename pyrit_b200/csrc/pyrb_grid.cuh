@@ -173,8 +173,13 @@ __global__ void __launch_bounds__(kBlock) k_grid_old(BuildDesc d) {
         val[k] = e < d.n_old ? __ldcs(d.old_vals + e) : 0u;
     }
 #pragma unroll
-    for (int k = 0; k < kBatch; ++k)
-        if (key[k] < d.grid_cells) d.grid[key[k]] = uint64_t(e0 + k * kBlock + 1) << 32 | val[k];
+    for (int k = 0; k < kBatch; ++k) {
+        // (of a key that comes twice the last entry is stored)
+        const uint32_t e = e0 + k * kBlock;
+        uint64_t next = __shfl_down_sync(kFull, key[k], 1);
+        if ((threadIdx.x & 31) == 31 && key[k] < d.grid_cells) next = e + 1 < d.n_old ? __ldg(d.old_keys + e + 1) : ~0ull;
+        if (key[k] < d.grid_cells && next != key[k]) d.grid[key[k]] = uint64_t(e + 1) << 32 | val[k];
+    }
 }
 
 // Entries -> cells: an atomic max of (entry index + 1) << 32 | value.

@@ -986,6 +986,18 @@ __device__ __forceinline__ void region_bases(const BuildDesc& d, uint32_t nz, ui
     if (lane == 0) { tbase[R] = tt; ibase[R] = tbs; }
 }
 
+// First voxel of every chunk of a chunk build on the grid (chunkFirst, gbuild.zig:237-242):
+// the voxels before its first cell, or 0xFFFFFFFF for a chunk without voxels. By the
+// threads of the kernel after the write pass.
+__device__ __forceinline__ void grid_chunk_first(const BuildDesc& d, uint32_t t0, uint32_t stride) {
+    if (!d.chunked || !(d.use_grid | d.use_bucket)) return;
+    const uint32_t total = d.counters[kCtrUnique];
+    for (uint32_t c = t0; c < d.seg_count; c += stride) {
+        const uint32_t v = d.chunk_vstart[c], next = c + 1 < d.seg_count ? d.chunk_vstart[c + 1] : total;
+        d.chunk_first[c] = next > v ? v : 0xFFFFFFFFu;
+    }
+}
+
 // Bricks grouped by the leaf-table region of their mask (BuildDesc::leaf_regions):
 // per tile, ranks within each region by shared-memory counters, one global cursor
 // reservation per region; the order inside a region does not matter (the owner is
@@ -996,6 +1008,7 @@ __global__ void __launch_bounds__(kBlock) k_leaf_part(BuildDesc d) {
     __shared__ uint32_t s_tb[kMaxLeafRegions + 1];
     const uint32_t B = min(d.counters[kCtrBricks], d.brick_bound);
     const uint32_t R = d.leaf_regions;
+    grid_chunk_first(d, blockIdx.x * kBlock + threadIdx.x, gridDim.x * kBlock);
     if (threadIdx.x < 32) region_bases(d, 0, 1, s_tb, s_base);  // s_base: each region's first brick
     for (uint32_t t0 = blockIdx.x * kBrickTile; t0 < B; t0 += gridDim.x * kBrickTile) {
         if (threadIdx.x < R) s_cnt[threadIdx.x] = 0;
@@ -1030,18 +1043,6 @@ __global__ void __launch_bounds__(kBlock) k_leaf_part(BuildDesc d) {
             }
         }
         __syncthreads();  // s_cnt and s_res are reused by the next tile
-    }
-}
-
-// First voxel of every chunk of a chunk build on the grid (chunkFirst, gbuild.zig:237-242):
-// the voxels before its first cell, or 0xFFFFFFFF for a chunk without voxels. By the
-// threads of the kernel after the write pass.
-__device__ __forceinline__ void grid_chunk_first(const BuildDesc& d, uint32_t t0, uint32_t stride) {
-    if (!d.chunked || !(d.use_grid | d.use_bucket)) return;
-    const uint32_t total = d.counters[kCtrUnique];
-    for (uint32_t c = t0; c < d.seg_count; c += stride) {
-        const uint32_t v = d.chunk_vstart[c], next = c + 1 < d.seg_count ? d.chunk_vstart[c + 1] : total;
-        d.chunk_first[c] = next > v ? v : 0xFFFFFFFFu;
     }
 }
 
