@@ -253,10 +253,10 @@ def kernel_roofline(stage_ms, st, n_in, n_u, leaves, key_bytes, peak, cells=0):
         return 20 * C + 28 * P + 4 * W
 
     for lv in range(2, 24):
-        nb, no = stage_ms.get("node_build:%d" % lv), stage_ms.get("node_own:%d" % lv)
-        if nb is None or no is None:
+        parts = [stage_ms.get("node_%s:%d" % (k, lv)) for k in ("build", "insert", "own")]
+        if None in parts:
             continue
-        add("node_dedup:%d" % lv, nb + no, node_bytes(lv))
+        add("node_dedup:%d" % lv, sum(parts), node_bytes(lv))
     return out
 
 
@@ -401,7 +401,7 @@ def run_ours(args):
     key_bytes = 4 if 3 * LOG2 + 1 <= 32 else 8
     peak, peak_kind = load_peaks()
     # the dominant kernel: the largest share of the build's stage time (a per-level
-    # node dedup is a pair of kernels, listed in "kernels" but not a candidate)
+    # node dedup is three kernels, listed in "kernels" but not a candidate)
     kernels = kernel_roofline(stage_ms, st, n_in, n_u, sizes["leaves"], key_bytes, peak,
                               cells=(1 << (3 * LOG2)) if st.sort_passes == 0 else 0)
     names = {"grid_scatter": "k_grid_scatter", "grid_count": "k_grid_count", "grid_write": "k_grid_write",
