@@ -87,7 +87,7 @@ constexpr uint64_t kGridCellsPerEntry = 4, kGridFreeCells = uint64_t(1) << 23;
 constexpr uint32_t kSmallLevelTiles = 296;
 constexpr uint64_t kGridMaxCells = uint64_t(1) << 33;
 // Up to this many compaction tiles the write pass adds up its own prefix (at most 256
-// group sums and 63 tile counts); larger grids take the 1024-thread scan kernel
+// group sums and 63 tile counts); larger grids take the scan kernel
 constexpr uint32_t kGridFoldTiles = 16384;
 // The brick buckets (pyrb_tuning.path = 3) need their brick counters (4 B per brick
 // position) well inside the L2: up to 2^24 bricks (64 MB, a 1024^3 volume). They are

@@ -16,16 +16,18 @@
 //   k_grid_scan     a cell is a voxel if its attribute word is not 0 (a cell no entry
 //   k_grid_write    reached is all zero; attribute 0 deletes). Tiles of 64 bricks of 64
 //                   cells: ballots give each brick's 64-bit mask directly. The count pass
-//                   writes every tile's voxels and non-empty bricks, one block scans
-//                   them, and the write pass reads the cells again and writes at the
-//                   final positions: the sorted unique keys and attributes, the brick
-//                   records and the per-chunk first voxel, exactly what the sort path's
-//                   k_unique writes. (A single pass with a decoupled look-back measured
-//                   barrier-bound: every block waited for its tile's look-back.)
+//                   writes every tile's voxels and non-empty bricks, the scan (large
+//                   grids) sums them up, and the write pass reads the cells again and
+//                   writes at the final positions: the sorted unique keys and attributes,
+//                   the brick records and the per-chunk first voxel, exactly what the
+//                   sort path's k_unique writes. (A single pass with a decoupled
+//                   look-back measured barrier-bound: every block waited for its tile's.)
+//   k_grid_old      the old voxels of an edit build, stored before the scatter.
 //
 // Bytes: 8 per cell for the zeroing, the atomics' line traffic and each of the two
 // reads, against 2 (kb + 4) per entry and pass of a sort: the grid wins while a chunk
-// has at most a few cells per entry (the host picks the path, see plan_build).
+// has at most a few cells per entry or the whole grid is small (the host picks the path,
+// see plan_build).
 #pragma once
 
 #include "pyrb_kernels.cuh"
@@ -113,7 +115,7 @@ __device__ __forceinline__ void for_tile_entries(const BuildDesc& d, const TileS
                 // the source voxels come in key order (x + 4y + 16z inside a brick): up to 8
                 // of them share a coarse cell, at distances 1, 4 and 16 in full bricks. Of a
                 // row's entries of a cell only the last can decide: those that a later one of
-                // the row replaces take no atomic (256^3 to 128^3: 50 -> 16 us)
+                // the row replaces take no atomic (256^3 to 128^3: 50 -> 21 us)
                 const uint32_t n1 = __shfl_down_sync(kFull, key, 1), n4 = __shfl_down_sync(kFull, key, 4),
                                n16 = __shfl_down_sync(kFull, key, 16);
                 const bool later = (lane < 31 && n1 == key) || (lane < 28 && n4 == key) || (lane < 16 && n16 == key);
@@ -156,10 +158,12 @@ __device__ __forceinline__ void for_tile_entries(const BuildDesc& d, const TileS
     }
 }
 
-// Old entries of a plain build -> cells. Their keys are sorted and unique and every entry
-// after them overrides them, so they are stored, before the others' atomics: the stores
-// are neighbours, while an atomic takes the L2 as long for each of their sectors as for
-// one on its own (5 M old voxels and 90,000 edits: 39 us by atomics, 30 like this with the edits' own pass).
+// Old entries of a plain build -> cells. Their keys are sorted (of equal ones the last
+// counts) and every entry after them overrides them, so they are stored, before the
+// others' atomics: the stores are neighbours, while an atomic takes the L2 as long for
+// each of their sectors as for one on its own (5 M old voxels and 90,000 edits: 39 us by
+// atomics, 30 like this with the edits' own pass). Where they turn out not to be sorted,
+// two stores may have met in a cell: the scatter settles it by atomics.
 __global__ void __launch_bounds__(kBlock) k_grid_old(BuildDesc d) {
     grid_dep_wait();
     constexpr int kBatch = 8;
@@ -177,7 +181,8 @@ __global__ void __launch_bounds__(kBlock) k_grid_old(BuildDesc d) {
         // (of a key that comes twice the last entry is stored)
         const uint32_t e = e0 + k * kBlock;
         uint64_t next = __shfl_down_sync(kFull, key[k], 1);
-        if ((threadIdx.x & 31) == 31 && key[k] < d.grid_cells) next = e + 1 < d.n_old ? __ldg(d.old_keys + e + 1) : ~0ull;
+        if ((threadIdx.x & 31) == 31) next = e + 1 < d.n_old ? __ldg(d.old_keys + e + 1) : ~0ull;
+        if (next < key[k] && e < d.n_old) d.counters[kCtrOldOrder] = 1u;
         if (key[k] < d.grid_cells && next != key[k]) d.grid[key[k]] = uint64_t(e + 1) << 32 | val[k];
     }
 }
@@ -192,6 +197,12 @@ __global__ void __launch_bounds__(kBlock) k_grid_scatter(BuildDesc d) {
     for_tile_entries(d, sp, [&](uint32_t e, uint32_t key, uint32_t val) {
         red_max_u64(cells + key, (uint64_t(e + 1) << 32) | val);
     });
+    if (d.one_seg && d.n_old && __ldcg(d.counters + kCtrOldOrder)) {  // (see k_grid_old)
+        for (uint64_t e = uint64_t(tile) * kBlock + threadIdx.x; e < d.n_old; e += uint64_t(gridDim.x) * kBlock) {
+            const uint64_t key = __ldg(d.old_keys + e);
+            if (key < d.grid_cells) red_max_u64(cells + key, ((e + 1) << 32) | __ldg(d.old_vals + e));
+        }
+    }
 }
 
 // The attribute words of a warp's kGridWarpBricks bricks: cells lane and 32 + lane of
@@ -337,7 +348,7 @@ __global__ void __launch_bounds__(kBlock, 8) k_grid_count(BuildDesc d) {
 
 // Pass 2 on its own (larger grids): blocks of kGridScanTile counts with a look-back
 // between them; both fields stay below 2^31, so they share a status word. (One block
-// over 547,000 tiles: 608 us of a 1024-chunk batch; now 10.)
+// over 547,000 tiles: 608 us of a 1024-chunk batch; now 16.)
 constexpr uint32_t kGridScanTile = kBlock * kGridScanPer;
 __global__ void __launch_bounds__(kBlock) k_grid_scan(BuildDesc d) {
     grid_dep_wait();

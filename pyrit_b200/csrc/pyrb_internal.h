@@ -21,6 +21,7 @@ constexpr int kCtrPrims = 5;
 constexpr int kCtrError = 6;
 constexpr int kCtrNeed = 7;        // largest generator count above the chunk capacity (world path)
 constexpr int kCtrCursor = 8;      // + lv: first node word of level lv (lv = 2..25)
+constexpr int kCtrOldOrder = 34;   // old keys of a grid build out of order
 constexpr int kCtrParents = 36;    // + lv: P_lv
 constexpr int kCtrUniqueLv = 64;   // + lv: U_lv
 constexpr int kCtrTiles = 96;      // dynamic tile counters, one per launch:

@@ -1562,7 +1562,7 @@ __global__ void __launch_bounds__(kBlock, NB == 1 ? 6 : 5) k_node_build(BuildDes
 // ~index in one 16-byte compare-and-swap. The words of every resident were written by the
 // kernel before, so nothing here needs an acquire or a release; they are compared where the
 // hashes are equal. Build, insert and owners of 256^3
-// noise take 18 + 12 + 13 us at level 2 (28,000 parents) and 11 + 10 + 11 at level 3 (4096);
+// noise take 17 + 14 + 12 us at level 2 (28,000 parents) and 12 + 12 + 10 at level 3 (4096);
 // with acquire-release inserts in the build kernel 32 + 15 and 32 + 11.
 constexpr int kProbes = 4;
 __global__ void __launch_bounds__(kBlock) k_node_insert(BuildDesc d, LevelDesc L) {

@@ -1,7 +1,8 @@
 """Leaf and node levels at the sizes where their work changes hands: the leaves and first
 levels of up to 4096 bricks in the one-block tail or in kernels of their own, tail levels
-of up to 1024 parents in shared memory or through global memory, and dedup tables whose
-bounds (from the input size) are far above the real counts. Byte for byte against the
+of up to 1024 parents in shared memory or through global memory, dedup tables whose
+bounds (from the input size) are far above the real counts, and old voxels that come
+twice or out of order. Byte for byte against the
 oracle restatement of the reference GPU algorithm."""
 import numpy as np
 import pytest
@@ -66,3 +67,28 @@ def test_one_large_chunk(path):
     finally:
         gpu_build.set_tuning(0, 0, 50, 0)
     assert_same_build(g, orc.gb_build_chunks(log2, 6, n, pts, offs), chunks=True, label=f"path {path}")
+
+
+@pytest.mark.parametrize("order", ["sorted", "twice", "rotated", "shuffled"])
+@pytest.mark.parametrize("n_new", [0, 1, 5000])
+def test_order_of_the_old_voxels(order, n_new):
+    """The last of equal keys counts, wherever it stands, and every edit after it."""
+    from pyrit_b200 import gpu_build
+    rng = np.random.default_rng(n_new)
+    log2, n = 6, 60_000
+    keys = np.sort(rng.choice(1 << 3 * log2, n, replace=False)).astype(np.uint64)
+    if order != "sorted":
+        keys = np.sort(keys[rng.integers(0, n, n)])
+    if order == "rotated":
+        keys = np.concatenate([keys[n // 3:], keys[: n // 2], np.array([1 << 3 * log2], np.uint64)])
+    if order == "shuffled":
+        keys = rng.permutation(keys)
+    vals = rng.integers(0, 200, len(keys)).astype(np.uint32)
+    ed = np.concatenate([rng.integers(0, 1 << log2, (n_new, 3)), rng.integers(0, 9, (n_new, 1))], 1).astype(np.uint32)
+    gpu_build.set_tuning(0, 0, 50, 2)
+    try:
+        g = gpu_build.build(log2, 4, dev(ed) if n_new else None, old_keys=dev(keys), old_vals=dev(vals),
+                            n_old=len(keys)).download()
+    finally:
+        gpu_build.set_tuning(0, 0, 50, 0)
+    assert_same_build(g, orc.gb_build(log2, 4, ed, old_keys=keys, old_vals=vals), label=order)
