@@ -85,6 +85,8 @@ std::atomic<uint32_t> g_path{kPathAuto};
 constexpr uint64_t kGridCellsPerEntry = 4, kGridFreeCells = uint64_t(1) << 23;
 // A node level takes tiles of one item per thread below this many large tiles (2 per SM)
 constexpr uint32_t kSmallLevelTiles = 296;
+// Blocks of the kernels that take tile after tile where the bounds ask for more: 8 per SM
+constexpr uint32_t kTileBlocks = 148u * 8u;
 constexpr uint64_t kGridMaxCells = uint64_t(1) << 33;
 // Up to this many compaction tiles the write pass adds up its own prefix (at most 256
 // group sums and 63 tile counts); larger grids take the scan kernel
@@ -270,9 +272,9 @@ uint32_t launch_levels(const BuildDesc& d, const std::vector<LevelDesc>& levels,
         launch(k_node_insert, std::max(std::min((L.parent_bound + kBlock - 1) / kBlock, 148u * 8u), 1u), kBlock, 0, st, d, L);
         prof.mark("node_insert", L.lv);
         if (L.own_it == 1)
-            launch(k_node_own<1>, L.own_tiles, kBlock, 0, st, d, L);
+            launch(k_node_own<1>, std::min(L.own_tiles, kTileBlocks), kBlock, 0, st, d, L);
         else
-            launch(k_node_own<kNodeIT>, L.own_tiles, kBlock, 0, st, d, L);
+            launch(k_node_own<kNodeIT>, std::min(L.own_tiles, kTileBlocks), kBlock, 0, st, d, L);
         prof.mark("node_own", L.lv);
         launches += 3;
         if (L.lv + 1 == d.rt_log2) {
@@ -878,7 +880,10 @@ uint32_t launch_plan(const Plan& p, const std::vector<LevelDesc>& levels, cudaSt
         prof.mark("leaf_part");
         ++launches;
         const uint32_t S = d.leaf_cap / d.leaf_regions, nz = (S + kZeroSlots - 1) / kZeroSlots;
-        launch(k_leaf_insert_regions, d.leaf_regions * (nz + 1) + (B + kInsTile - 1) / kInsTile, kBlock, 0, st, d);
+        // bricks bounded by the entries, not by the volume: a brick holds several entries, so
+        // most of the bound's tiles are not there
+        const uint32_t tiles = d.leaf_regions * (nz + 1) + (B + kInsTile - 1) / kInsTile;
+        launch(k_leaf_insert_regions, B == p.nmax ? std::min(tiles, kTileBlocks) : tiles, kBlock, 0, st, d);
     } else {
         launch(k_leaf_insert, leaf_insert_grid(d), kBlock, 0, st, d);
     }

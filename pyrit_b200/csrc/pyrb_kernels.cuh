@@ -1108,17 +1108,10 @@ constexpr uint32_t kZeroSlots = PYRB_ZERO_SLOTS;  // slots a clearing tile clear
 constexpr int kInsPerThread = PYRB_INS_PER_THREAD;
 constexpr uint32_t kInsTile = kInsPerThread * kBlock;  // bricks an insert tile takes
 
-__global__ void __launch_bounds__(kBlock) k_leaf_insert_regions(BuildDesc d) {
-    grid_dep_wait();
-    __shared__ uint32_t s_tile;
-    __shared__ uint32_t s_tbase[kMaxLeafRegions + 1], s_ibase[kMaxLeafRegions + 1];
-    const uint32_t B = min(d.counters[kCtrBricks], d.brick_bound);
-    const LeafTable t = leaf_table_of(d, B);
-    const uint32_t R = d.leaf_regions, S = t.slots / R, smask = S - 1;
-    const uint32_t nz = (S + kZeroSlots - 1) / kZeroSlots;
-    if (threadIdx.x < 32) region_bases(d, nz, kInsTile, s_tbase, s_ibase);
-    const uint32_t tile = dyn_tile(d.counters, kTileLeafInsert, &s_tile);  // its barrier publishes s_tbase
-    if (tile >= s_tbase[R]) return;
+__device__ __forceinline__ void leaf_region_tile(const BuildDesc& d, const LeafTable& t, const uint32_t B,
+                                                 const uint32_t nz, const uint32_t* s_tbase, const uint32_t* s_ibase,
+                                                 const uint32_t tile) {
+    const uint32_t S = t.slots / d.leaf_regions, smask = S - 1;
     uint32_t r = 0;
     while (s_tbase[r + 1] <= tile) ++r;
     const uint32_t k = tile - s_tbase[r];
@@ -1173,6 +1166,27 @@ __global__ void __launch_bounds__(kBlock) k_leaf_insert_regions(BuildDesc d) {
         }
         // one byte per brick that became an owner: scattered, but the array stays in L2
         if (v[q] && (s[q] & kInstalled)) d.binst[b[q]] = 1;
+    }
+}
+
+// A launch of fewer blocks than there may be tiles has them take tile after tile (a block
+// without a tile still takes some 2 us: 4096^3 surface, bounds of 37,000 tiles and 7000
+// real ones, 70 -> 37 us). Where the bound is met, a block per tile is the faster one
+// (1024^3 at 15 %, 73,000 tiles: 660 us, 725 in a loop).
+__global__ void __launch_bounds__(kBlock) k_leaf_insert_regions(BuildDesc d) {
+    grid_dep_wait();
+    __shared__ uint32_t s_tile;
+    __shared__ uint32_t s_tbase[kMaxLeafRegions + 1], s_ibase[kMaxLeafRegions + 1];
+    const uint32_t B = min(d.counters[kCtrBricks], d.brick_bound);
+    const LeafTable t = leaf_table_of(d, B);
+    const uint32_t nz = (t.slots / d.leaf_regions + kZeroSlots - 1) / kZeroSlots;
+    if (threadIdx.x < 32) region_bases(d, nz, kInsTile, s_tbase, s_ibase);
+    while (true) {
+        const uint32_t tile = dyn_tile(d.counters, kTileLeafInsert, &s_tile);  // its barrier publishes s_tbase
+        const uint32_t tiles = s_tbase[d.leaf_regions];
+        if (tile >= tiles) return;
+        leaf_region_tile(d, t, B, nz, s_tbase, s_ibase, tile);
+        if (tiles <= gridDim.x) return;
     }
 }
 
@@ -1629,14 +1643,12 @@ __global__ void __launch_bounds__(kBlock) k_node_insert(BuildDesc d, LevelDesc L
 // owner test, so that the tile takes two dependent round trips before its look-back.
 template <int NIT>
 __device__ __forceinline__ void node_own_tile(const BuildDesc& d, const LevelDesc& L, const uint32_t tile,
-                                              const uint32_t parents, const uint32_t cursor) {
+                                              const uint32_t P, const uint32_t cursor) {
     __shared__ uint64_t s_scan[2 * kWarps + 2];
     __shared__ uint64_t s_base;
     const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint32_t P = min(parents, L.parent_bound);
     constexpr uint32_t kTile = kBlock * NIT;
     const uint32_t ntiles = (P + kTile - 1) / kTile;
-    if (tile >= ntiles) return;
     const uint32_t wstart = tile * kTile + warp * 32 * NIT;
     uint32_t len[NIT], slot[NIT];
     uint32_t w1[NIT == 1 ? kNodeStride : 1];  // NIT == 1: the parent's words
@@ -1729,14 +1741,22 @@ __device__ __forceinline__ void node_own_tile(const BuildDesc& d, const LevelDes
     }
 }
 
+// Fewer blocks than there may be tiles: they take tile after tile (4096^3 surface, levels 2
+// to 5: 25 + 18 + 18 + 14 -> 20 + 14 + 14 + 13 us; 1024^3 level 2: 154 -> 144).
 template <int NIT>
 __global__ void __launch_bounds__(kBlock) k_node_own(BuildDesc d, LevelDesc L) {
     grid_dep_wait();
     __shared__ uint32_t s_tile[3];
     uint32_t parents, cursor;
-    const uint32_t tile = dyn_tile_and(d.counters, L.tile_ctr_own, kCtrParents + L.lv, kCtrCursor + L.lv, s_tile,
-                                       &parents, &cursor);
-    node_own_tile<NIT>(d, L, tile, parents, cursor);
+    while (true) {
+        const uint32_t tile = dyn_tile_and(d.counters, L.tile_ctr_own, kCtrParents + L.lv, kCtrCursor + L.lv, s_tile,
+                                           &parents, &cursor);
+        const uint32_t P = min(parents, L.parent_bound);
+        const uint32_t ntiles = (P + kBlock * NIT - 1) / (kBlock * NIT);
+        if (tile >= ntiles) return;
+        node_own_tile<NIT>(d, L, tile, P, cursor);
+        if (ntiles <= gridDim.x) return;
+    }
 }
 
 // Empty levels still have to pass the cursor on.

@@ -38,10 +38,10 @@ def test_tail_limits(log2, rt, n, per_parent):
     assert_same_build(g, orc.gb_build(log2, rt, pts), label=f"{n} {per_parent}")
 
 
-@pytest.mark.parametrize("edge", [3, 40])
+@pytest.mark.parametrize("edge", [3, 40, 300])
 def test_tables_far_above_the_real_counts(edge):
     """2.2 M entries of a 2^11 volume inside a cube of `edge` bricks: bounds of millions of
-    bricks (a leaf table of regions), a few or some ten thousand real ones."""
+    bricks (a leaf table of regions), a few, some ten thousand or as many real ones."""
     from pyrit_b200 import gpu_build
     rng = np.random.default_rng(edge)
     n = 2_200_000
