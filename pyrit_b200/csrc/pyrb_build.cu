@@ -85,6 +85,11 @@ std::atomic<uint32_t> g_path{kPathAuto};
 constexpr uint64_t kGridCellsPerEntry = 4, kGridFreeCells = uint64_t(1) << 23;
 // A node level takes tiles of one item per thread below this many large tiles (2 per SM)
 constexpr uint32_t kSmallLevelTiles = 296;
+// Entries with 64-bit keys from which their sort tiles have 4096 of them. Larger tiles take
+// 2 to 3 us off each of the four or more passes (2.9 M keys 38.8 -> 36.8, 7.4 M 84 -> 81) and
+// cost the encode 0 to 4 us, which is what they save below some 2 M (1.3 M: 23.0 -> 22.9, encode
+// 21.5 -> 25.5)
+constexpr uint64_t kLargeTiles64 = uint64_t(1) << 21;
 // Blocks of the kernels that take tile after tile where the bounds ask for more: 8 per SM
 constexpr uint32_t kTileBlocks = 148u * 8u;
 constexpr uint64_t kGridMaxCells = uint64_t(1) << 33;
@@ -355,11 +360,12 @@ void fill_stats(const uint32_t* ctr, const uint32_t* meta) {
     g_stats = s;
 }
 
-// Sort tiles of IT * kBlock entries. Tiles of 8192 entries (IT = 32) are sorted by
-// 512-thread blocks of 16 entries per thread and de-duplicated in two 4096-entry parts.
+// Sort tiles of IT * kBlock entries. Tiles of 8192 entries (IT = 32; of 64-bit keys 4096)
+// are sorted by 512-thread blocks of 16 (8) entries per thread and de-duplicated in two
+// parts.
 template <int RB, int IT, typename KeyT = uint32_t>
 cudaError_t launch_sort(const BuildDesc& d, cudaStream_t st, Prof& prof) {
-    constexpr int NT = IT > 16 ? 2 * kBlock : kBlock, SIT = IT * kBlock / NT;
+    constexpr int NT = IT * sizeof(KeyT) > 64 ? 2 * kBlock : kBlock, SIT = IT * kBlock / NT;
     constexpr int UIT = SIT < kUniqIT ? SIT : kUniqIT;
     constexpr uint32_t parts = uint32_t(IT / UIT);  // unique tiles per sort tile
     const size_t hist_smem = size_t(d.passes) * (1u << RB) * 4;
@@ -384,9 +390,10 @@ cudaError_t launch_sort(const BuildDesc& d, cudaStream_t st, Prof& prof) {
     return cudaGetLastError();
 }
 
-// 64-bit sort keys (edges above 2^10): one digit width and tile, 8 bits x 2048 keys.
+// 64-bit sort keys (edges above 2^10): 8-bit digits, tiles of 2048 or 4096 keys.
 cudaError_t launch_sort_any(uint32_t rb, uint32_t it, const BuildDesc& d, cudaStream_t st, Prof& prof) {
-    if (3 * d.log2 + 1 > 32) return launch_sort<8, 8, uint64_t>(d, st, prof);
+    if (3 * d.log2 + 1 > 32)
+        return it == 16 ? launch_sort<8, 16, uint64_t>(d, st, prof) : launch_sort<8, 8, uint64_t>(d, st, prof);
     if (rb == 9 && it == 16) return launch_sort<9, 16>(d, st, prof);
     if (rb == 9 && it == 8) return launch_sort<9, 8>(d, st, prof);
     if (rb == 9 && it == 4) return launch_sort<9, 4>(d, st, prof);
@@ -449,7 +456,7 @@ struct Plan {
 };
 
 // Digit width, tile and load factor of a build: the fixed tuning given, else the
-// library's current tuning (64-bit keys: 8-bit digits on 2048-key tiles).
+// library's current tuning (64-bit keys: 8-bit digits on 2048- or 4096-key tiles).
 struct Tune {
     uint32_t rb, tile_keys, lf, path;
 };
@@ -495,7 +502,7 @@ pyrb_result plan_build(const Job& job, const Tune* fixed, Plan& p) {
     const uint32_t n = p.n = uint32_t(n64);
     const uint32_t nmax = p.nmax = std::max(n, 1u);
 
-    // tuning (64-bit keys use 8-bit digits and 2048-key tiles)
+    // tuning (64-bit keys use 8-bit digits on tiles of 2048 or 4096 keys)
     uint32_t rb, tile_keys, lf, path;
     if (fixed) {
         rb = fixed->rb;
@@ -504,7 +511,7 @@ pyrb_result plan_build(const Job& job, const Tune* fixed, Plan& p) {
         path = fixed->path;
     } else {
         rb = p.key64 ? 8u : g_radix_bits.load();
-        tile_keys = p.key64 ? 2048u : g_tile_keys.load();
+        tile_keys = !p.key64 ? g_tile_keys.load() : nmax >= kLargeTiles64 ? 4096u : 2048u;
         if (rb == 0) {
             auto_tuning(lb - 6, &rb, &tile_keys);
             // chunks that a 4096-entry tile (nearly) holds would leave 8192-entry ones half empty
@@ -580,7 +587,8 @@ pyrb_result plan_build(const Job& job, const Tune* fixed, Plan& p) {
     }
     if (words >= (uint64_t(1) << 32)) return fail(PYRB_ERROR_INVALID_ARGUMENT, "node buffer bound exceeds 2^32 words");
     d.brick_bound = B;
-    d.brick_tiles = d.sort_tiles * std::max(1u, tile_keys / uint32_t(kBlock * kUniqIT));  // the unique tiles
+    // the unique tiles (launch_sort)
+    d.brick_tiles = d.sort_tiles * std::max(1u, tile_keys / (p.key64 ? 2048u : uint32_t(kBlock * kUniqIT)));
     d.leafown_tiles = std::max((B + kBrickTile - 1) / kBrickTile, 1u);
     if ((uint64_t(B) * 100 + lf - 1) / lf > (uint64_t(1) << 31))
         return fail(PYRB_ERROR_INVALID_ARGUMENT, "brick bound exceeds the leaf table's 2^31 slots");
