@@ -111,7 +111,9 @@ __device__ __forceinline__ void for_tile_entries(const BuildDesc& d, const TileS
 #pragma unroll
             for (int k = 0; k < kScatterBatch; ++k) {
                 const uint32_t idx = base + k * kBlock + threadIdx.x;
-                const uint32_t key = idx < sp.count ? uint32_t(coarse_key(src[k], d.shift)) : 0xFFFFFFFFu;
+                // (a source key outside the volume has no cell: compared before it is cut to 32 bits)
+                const uint64_t coarse = coarse_key(src[k], d.shift);
+                const uint32_t key = idx < sp.count && coarse < d.grid_cells ? uint32_t(coarse) : 0xFFFFFFFFu;
                 // the source voxels come in key order (x + 4y + 16z inside a brick): up to 8
                 // of them share a coarse cell, at distances 1, 4 and 16 in full bricks. Of a
                 // row's entries of a cell only the last can decide: those that a later one of
@@ -119,7 +121,7 @@ __device__ __forceinline__ void for_tile_entries(const BuildDesc& d, const TileS
                 const uint32_t n1 = __shfl_down_sync(kFull, key, 1), n4 = __shfl_down_sync(kFull, key, 4),
                                n16 = __shfl_down_sync(kFull, key, 16);
                 const bool later = (lane < 31 && n1 == key) || (lane < 28 && n4 == key) || (lane < 16 && n16 == key);
-                if (idx < sp.count && !later) f(sp.start + idx, key, val[k]);
+                if (key != 0xFFFFFFFFu && !later) f(sp.start + idx, key, val[k]);
             }
         }
         return;

@@ -189,12 +189,19 @@ __device__ __forceinline__ void encode_voxel(uint4 v, uint32_t log2, uint32_t lb
     }
 }
 
+// A key that the caller gives (old voxels, the source of a downsample), compared before it
+// is cut to KeyT: one outside the volume becomes the invalid key, as a coordinate does.
+template <typename KeyT>
+__device__ __forceinline__ KeyT given_key(uint64_t key, uint32_t lb) {
+    return key >> lb ? KeyT(1) << lb : KeyT(key);
+}
+
 template <typename KeyT>
 __device__ __forceinline__ void load_raw(const BuildDesc& d, uint32_t seg, uint32_t j, KeyT& key, uint32_t& val) {
     switch (d.mode) {
         case kModePlain:
             if (j < d.n_old) {
-                key = KeyT(__ldg(d.old_keys + j));
+                key = given_key<KeyT>(__ldg(d.old_keys + j), d.lb);
                 val = __ldg(d.old_vals + j);
             } else {
                 encode_voxel(__ldg(d.voxels + (j - d.n_old)), d.log2, d.lb, key, val);
@@ -219,7 +226,7 @@ __device__ __forceinline__ void load_raw(const BuildDesc& d, uint32_t seg, uint3
             break;
         }
         default: {  // downsample (gbuild.zig:262-274): coarse key of the source voxel
-            key = KeyT(coarse_key(__ldg(d.src_keys + j), d.shift));
+            key = given_key<KeyT>(coarse_key(__ldg(d.src_keys + j), d.shift), d.lb);
             val = __ldg(d.src_vals + j);
             break;
         }

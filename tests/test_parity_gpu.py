@@ -437,3 +437,49 @@ def test_old_voxels_and_edits_at_tile_edges(gb, n_old, n_new):
     g = gb.build(5, 3, dev(ed) if n_new else None, old_keys=dev(old.keys), old_vals=dev(old.attrs),
                  n_old=n_old).download()
     assert_same_build(g, orc.gb_build(5, 3, ed, old_keys=old.keys, old_vals=old.attrs), label=f"{n_old}+{n_new}")
+
+
+# Keys outside the volume: the next x, y or z beyond it, the keys of the next chunk of a
+# batch, one more 32-bit range (the low word is a valid key) and the highest bits.
+def _keys_outside(log2, inside):
+    lb = 3 * log2
+    out = [1 << (lb + b) for b in range(4)] + [(1 << 33) + int(inside[0]), (5 << lb) + int(inside[-1]), 1 << 62,
+                                               (1 << 63) + int(inside[0]), (1 << 64) - 1]
+    return np.array([k for k in out if k >> lb], np.uint64)
+
+
+def _mixed_in(rng, keys, vals, outside, order):
+    """The keys outside behind the valid ones (sorted, as a later chunk's are) or anywhere."""
+    k = np.concatenate([keys, outside, outside])
+    v = np.concatenate([vals, rng.integers(0, 9, 2 * len(outside)).astype(np.uint32)])
+    if order == "behind":
+        p = np.argsort(k, kind="stable")
+    else:
+        at = np.sort(rng.choice(len(k), len(keys), replace=False))
+        p = np.empty(len(k), np.int64)
+        p[np.setdiff1d(np.arange(len(k)), at)] = np.arange(len(keys), len(k))
+        p[at] = np.arange(len(keys))
+    return k[p], v[p]
+
+
+@pytest.mark.parametrize("order", ["behind", "anywhere"])
+@pytest.mark.parametrize("log2,shift,n_src", [(4, 1, 300), (6, 1, 5000), (6, 3, 5000), (12, 1, 3000)])
+def test_downsample_drops_source_keys_outside_the_volume(gb, log2, shift, n_src, order):
+    rng = np.random.default_rng(log2 + shift)
+    pts = np.concatenate([rng.integers(0, 1 << log2, (n_src, 3)), rng.integers(1, 9, (n_src, 1))], 1).astype(np.uint32)
+    src = orc.gb_build(log2, 3, pts)
+    keys, vals = _mixed_in(rng, src.keys, src.attrs, _keys_outside(log2, src.keys), order)
+    g = gb.downsample(log2, 3, dev(keys), dev(vals), len(keys), shift).download()
+    assert_same_build(g, orc.gb_downsample(log2, 3, src.keys, src.attrs, shift), label=f"{log2} {shift} {order}")
+
+
+@pytest.mark.parametrize("order", ["behind", "anywhere"])
+@pytest.mark.parametrize("log2,n_old,n_new", [(3, 100, 0), (6, 5000, 400), (11, 3000, 400)])
+def test_old_keys_outside_the_volume_are_dropped(gb, log2, n_old, n_new, order):
+    rng = np.random.default_rng(log2)
+    pts = np.concatenate([rng.integers(0, 1 << log2, (n_old, 3)), rng.integers(1, 9, (n_old, 1))], 1).astype(np.uint32)
+    ed = np.concatenate([rng.integers(0, 1 << log2, (n_new, 3)), rng.integers(0, 9, (n_new, 1))], 1).astype(np.uint32)
+    old = orc.gb_build(log2, 3, pts)
+    keys, vals = _mixed_in(rng, old.keys, old.attrs, _keys_outside(log2, old.keys), order)
+    g = gb.build(log2, 3, dev(ed) if n_new else None, old_keys=dev(keys), old_vals=dev(vals), n_old=len(keys)).download()
+    assert_same_build(g, orc.gb_build(log2, 3, ed, old_keys=old.keys, old_vals=old.attrs), label=f"{log2} {order}")
