@@ -342,6 +342,10 @@ PYRB_API pyrb_result pyrb_path_edit(const pyrb_exec* e, uint64_t nodes, uint64_t
  * edge 2^log2_size, or, when chunk_log2 (host u32[count]) is given, of edges
  * 2^chunk_log2[c] (a pyrb_build_batch; log2_size is ignored); rt_log2_req as the build
  * takes it (it sizes the prim outputs). Uses the current tuning.
+ * With the automatic path, scratch includes the cells of the grid (8 bytes each) where the
+ * build would use one; the 2^23 cells that a sparse small volume may take beyond 4 per entry
+ * are up to 64 MB, whatever its entries. Where the allocator refuses such a build's scratch or
+ * outputs, the build sorts instead, in the memory that is reported with pyrb_tuning.path = 1.
  * scratch_bytes: freed when the build returns; output_bytes: the six output buffers.
  * The reference bounds its build scratch with a counting Exec (tests/cpu_test.zig:1559-1629). */
 PYRB_API pyrb_result pyrb_build_memory(uint32_t log2_size, uint32_t rt_log2_req, uint32_t count,
@@ -370,8 +374,8 @@ PYRB_API pyrb_result pyrb_selftest_wait_limit(const pyrb_exec* e, uint32_t which
  * stream; whenever one completes, the requests that arrived meanwhile form the next
  * pyrb_build_batch (at most max_batch_requests and max_batch_entries voxels + edits;
  * a larger request runs alone). All scratch and results live in one device arena of
- * budget_bytes: a batch is admitted when the build's exact need (pyrb_build_memory)
- * fits, after evicting the least recently completed batches (those whose results were
+ * budget_bytes: a batch is admitted when the build's need (pyrb_build_memory; the
+ * sort's for sparse small chunks) fits, after evicting the least recently completed batches (those whose results were
  * all released first). A result stays valid until released or, when the arena is
  * full, evicted: copy out what must outlive that. Each result is bit-identical to the
  * same chunk built alone. */

@@ -461,7 +461,9 @@ struct Tune {
     uint32_t rb, tile_keys, lf, path;
 };
 
-pyrb_result plan_build(const Job& job, const Tune* fixed, Plan& p) {
+// lean: without the cells that a small volume is given beyond kGridCellsPerEntry (the plan of
+// a build whose allocator has no room for them).
+pyrb_result plan_build(const Job& job, const Tune* fixed, Plan& p, bool lean = false) {
     const uint32_t log2 = job.log2;
     if (log2 < 3 || log2 > 20) return fail(PYRB_ERROR_INVALID_ARGUMENT, "log2_size must lie in [3, 20] (got %u)", log2);
     const uint32_t lb = 3 * log2;
@@ -524,7 +526,8 @@ pyrb_result plan_build(const Job& job, const Tune* fixed, Plan& p) {
     uint64_t grid_cells = 0;
     for (uint32_t l = 3; l <= log2 && !p.key64; ++l) grid_cells += per_log2[l] << (3 * l);
     if (!p.key64 && grid_cells <= kGridMaxCells)
-        p.grid = path == kPathGrid || (path == kPathAuto && grid_cells <= kGridCellsPerEntry * nmax + kGridFreeCells);
+        p.grid = path == kPathGrid ||
+                 (path == kPathAuto && grid_cells <= kGridCellsPerEntry * nmax + (lean ? 0 : kGridFreeCells));
     if (!p.key64 && !p.grid && (grid_cells >> 6) <= kBucketMaxBricks)
         p.bucket = path == kPathBucket;
     if (p.grid || p.bucket) tile_keys = 4096;  // the scatter's tiles over the entries
@@ -922,22 +925,37 @@ pyrb_result run_build(const pyrb_exec* e, const Job& job, pyrb_built* out, uint3
     Mem mem{e, st};
 
     // ---- allocations
-    uint64_t scratch = mem.get(p.scratch_bytes);
-    if (!scratch) return fail(PYRB_ERROR_OUT_OF_MEMORY, "device memory for the build scratch (%llu bytes)", (unsigned long long)p.scratch_bytes);
-    uint64_t outs[6] = {};
-    bool ok = true;
-    for (int i = 0; i < 6; ++i) ok = (outs[i] = mem.get(p.out_size[i])) != 0 && ok;
+    uint64_t scratch = 0, outs[6] = {};
     auto release_outputs = [&] {
-        for (uint64_t q : outs) mem.put(q);
+        for (uint64_t& q : outs) {
+            mem.put(q);
+            q = 0;
+        }
     };
     auto cleanup = [&] {
         release_outputs();
         mem.put(scratch);
+        scratch = 0;
     };
-    if (!ok) {
-        cleanup();
-        return fail(PYRB_ERROR_OUT_OF_MEMORY, "device memory for the build outputs");
+    auto allocate = [&]() -> const char* {  // nullptr, or what there was no memory for
+        const char* none = (scratch = mem.get(p.scratch_bytes)) ? nullptr : "scratch";
+        for (int i = 0; i < 6 && !none; ++i)
+            if (!(outs[i] = mem.get(p.out_size[i]))) none = "outputs";
+        if (none) cleanup();
+        return none;
+    };
+    const char* none = allocate();
+    if (none && p.grid) {
+        // no room for the cells of a sparse small volume: the sort does without them
+        Plan q;
+        if (plan_build(job, nullptr, q, true) == PYRB_OK && !q.grid) {
+            p = q;
+            none = allocate();
+        }
     }
+    if (none)
+        return fail(PYRB_ERROR_OUT_OF_MEMORY, "device memory for the build %s (%llu bytes)", none,
+                    (unsigned long long)(*none == 's' ? p.scratch_bytes : p.out_bytes()));
     std::vector<LevelDesc> levels;
     bind_plan(p, scratch, outs, job, levels);
     const BuildDesc& d = p.d;
@@ -1009,6 +1027,42 @@ pyrb_result run_build(const pyrb_exec* e, const Job& job, pyrb_built* out, uint3
 }
 
 }  // namespace
+
+namespace pyrb {
+// pyrb_build_memory; least: of a build whose allocator has no room for the cells of a sparse
+// small volume (see run_build).
+pyrb_result build_memory(uint32_t log2_size, uint32_t rt_log2_req, uint32_t count, const uint32_t* chunk_log2,
+                         uint64_t entries, bool least, uint64_t* scratch_bytes, uint64_t* output_bytes) {
+    if (count == 0) return fail(PYRB_ERROR_INVALID_ARGUMENT, "count is 0");
+    if (entries >= (uint64_t(1) << 31))
+        return fail(PYRB_ERROR_INVALID_ARGUMENT, "too many entries for one build (%llu)", (unsigned long long)entries);
+    Job j;
+    j.K = count;
+    j.rt_req = rt_log2_req;
+    if (chunk_log2) {
+        uint32_t lmax = 0;
+        for (uint32_t c = 0; c < count; ++c) lmax = std::max(lmax, chunk_log2[c]);
+        j.mode = kModeBatch;
+        j.log2 = lmax;
+        j.chunk_log2_host = chunk_log2;
+        j.voxel_total = uint32_t(entries);
+    } else if (count > 1) {
+        j.mode = kModeChunks;
+        j.log2 = log2_size;
+        j.total = uint32_t(entries);
+    } else {
+        j.mode = kModePlain;
+        j.log2 = log2_size;
+        j.n_new = uint32_t(entries);
+    }
+    Plan p;
+    pyrb_result r = plan_build(j, nullptr, p, least);
+    if (r != PYRB_OK) return r;
+    if (scratch_bytes) *scratch_bytes = p.scratch_bytes;
+    if (output_bytes) *output_bytes = p.out_bytes();
+    return PYRB_OK;
+}
+}  // namespace pyrb
 
 namespace pyrb {
 // The calling thread's error message, for the library's other translation units.
@@ -1529,34 +1583,7 @@ PYRB_API pyrb_result pyrb_path_edit(const pyrb_exec* e, uint64_t nodes, uint64_t
 PYRB_API pyrb_result pyrb_build_memory(uint32_t log2_size, uint32_t rt_log2_req, uint32_t count,
                                        const uint32_t* chunk_log2, uint64_t entries, uint64_t* scratch_bytes,
                                        uint64_t* output_bytes) {
-    if (count == 0) return fail(PYRB_ERROR_INVALID_ARGUMENT, "count is 0");
-    if (entries >= (uint64_t(1) << 31))
-        return fail(PYRB_ERROR_INVALID_ARGUMENT, "too many entries for one build (%llu)", (unsigned long long)entries);
-    Job j;
-    j.K = count;
-    j.rt_req = rt_log2_req;
-    if (chunk_log2) {
-        uint32_t lmax = 0;
-        for (uint32_t c = 0; c < count; ++c) lmax = std::max(lmax, chunk_log2[c]);
-        j.mode = kModeBatch;
-        j.log2 = lmax;
-        j.chunk_log2_host = chunk_log2;
-        j.voxel_total = uint32_t(entries);
-    } else if (count > 1) {
-        j.mode = kModeChunks;
-        j.log2 = log2_size;
-        j.total = uint32_t(entries);
-    } else {
-        j.mode = kModePlain;
-        j.log2 = log2_size;
-        j.n_new = uint32_t(entries);
-    }
-    Plan p;
-    pyrb_result r = plan_build(j, nullptr, p);
-    if (r != PYRB_OK) return r;
-    if (scratch_bytes) *scratch_bytes = p.scratch_bytes;
-    if (output_bytes) *output_bytes = p.out_bytes();
-    return PYRB_OK;
+    return pyrb::build_memory(log2_size, rt_log2_req, count, chunk_log2, entries, false, scratch_bytes, output_bytes);
 }
 
 PYRB_API uint32_t pyrb_last_capacity_need(void) { return g_capacity_need; }

@@ -15,9 +15,10 @@
 //   so requests that arrive while others build join the next batch;
 // * all scratch and all results are sub-allocated from one device arena of
 //   budget_bytes (first fit with coalescing, the idea of src/range_alloc.zig:25-58).
-//   A batch is admitted when its exact need (the build's own bounds,
-//   pyrb_build_memory) fits into the largest free range, after evicting the least
-//   recently completed results (released ones first);
+//   A batch is admitted when its need (the build's own bounds; the sort's for sparse
+//   small chunks, whose cells are taken only where there is room for them) fits into
+//   the largest free range, after evicting the least recently completed results
+//   (released ones first);
 // * pyrb_server_poll hands out finished results (device buffers of the batch and the
 //   chunk's root, first voxel and prim); latency = submit -> the worker saw the batch
 //   complete (host clock).
@@ -43,8 +44,10 @@
 
 #include "pyrit_b200.h"
 
-namespace pyrb {
-pyrb_result set_error(pyrb_result r, const char* msg);  // pyrb_build.cu
+namespace pyrb {  // pyrb_build.cu
+pyrb_result set_error(pyrb_result r, const char* msg);
+pyrb_result build_memory(uint32_t log2_size, uint32_t rt_log2_req, uint32_t count, const uint32_t* chunk_log2,
+                         uint64_t entries, bool least, uint64_t* scratch_bytes, uint64_t* output_bytes);
 }
 
 namespace {
@@ -290,9 +293,9 @@ struct pyrb_server {
             if (m) std::memcpy(s->h_edits + uint64_t(s->h_eoff[k]) * 4, r.edits.data(), uint64_t(m) * 16);
             s->h_eoff[k + 1] = s->h_eoff[k] + m;
         }
-        // admission: the build's exact need must fit the largest free range
+        // admission: what the build cannot do without must fit the largest free range
         uint64_t scratch = 0, outs = 0;
-        if (pyrb_build_memory(0, cfg.rt_log2, K, s->log2.data(), entries, &scratch, &outs) != PYRB_OK) return false;
+        if (pyrb::build_memory(0, cfg.rt_log2, K, s->log2.data(), entries, true, &scratch, &outs) != PYRB_OK) return false;
         const uint64_t need = scratch + outs + 8 * Arena::kAlign;
         while (arena.largest_free() < need && evict_one()) {
         }

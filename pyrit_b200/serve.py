@@ -101,7 +101,7 @@ class _ArenaView:
 class ChunkServer:
     """Continuous batching over a device-resident chunk pool, by the library's native
     served loop (pyrb_server_*: a worker thread, a first-fit device arena of
-    `budget_bytes` for all scratch and results, admission by the build's exact memory
+    `budget_bytes` for all scratch and results, admission by the build's memory
     need, LRU eviction). This class submits requests at their arrival times, polls the
     finished results and keeps the statistics."""
 

@@ -7,7 +7,9 @@
 * The world path never cuts a chunk off: a generator count above the capacity is
   reported as PYRB_ERROR_CAPACITY with the count needed (the reference grows the
   capacity and generates again, src/world.zig:968-996); the retry with the grown
-  capacity builds what the reference's worldedit + buildChunks would."""
+  capacity builds what the reference's worldedit + buildChunks would.
+* A caller's own allocator whose budget holds the sort's scratch but not the cells that
+  a sparse small build would rather use still gets its build."""
 import ctypes
 
 import numpy as np
@@ -85,3 +87,56 @@ def test_chunk_over_capacity_is_reported_and_the_retry_builds_everything():
         packed[c * cap2:c * cap2 + oc[c]] = ov[c * cap2:c * cap2 + oc[c]]
     o = orc.gb_build_chunks(log2, 4, cap2, packed, offs)
     assert_same_build(g, o, chunks=True, label="grown capacity")
+
+
+class _Arena:
+    """A caller's allocator: 256-byte steps through one block, nothing beyond its budget."""
+
+    def __init__(self, budget):
+        import torch
+        self.block = torch.zeros(budget, dtype=torch.uint8, device="cuda")
+        self.budget, self.used, self.live, self.refused = budget, 0, {}, 0
+        self.ex = native.Exec(stream=ctypes.c_void_p(torch.cuda.current_stream().cuda_stream),
+                              alloc=native.ALLOC_FN(self.alloc), free=native.FREE_FN(self.free))
+
+    def alloc(self, _, n):
+        n = (int(n) + 255) // 256 * 256
+        if self.used + n > self.budget:
+            self.refused += 1
+            return 0
+        p = self.block.data_ptr() + self.used
+        self.live[p] = n
+        self.used += n
+        return p
+
+    def free(self, _, p):
+        del self.live[p]
+        if not self.live:
+            self.used = 0
+
+
+@pytest.mark.parametrize("room", ["scratch", "outputs"])
+@pytest.mark.parametrize("log2,n", [(7, 1000), (6, 40)])
+def test_a_budget_for_the_sort_is_enough(log2, n, room):
+    """The budget ends below the cells (room for the sort's scratch and the outputs only), or
+    between the cells and the outputs behind them."""
+    from pyrit_b200 import gpu_build
+    rng = np.random.default_rng(n)
+    pts = np.concatenate([rng.integers(0, 1 << log2, (n, 3)), rng.integers(1, 9, (n, 1))], 1).astype(np.uint32)
+    grid, outs = gpu_build.build_memory(log2, n, rt_log2_req=4)
+    gpu_build.set_tuning(0, 0, 50, native.PATH_SORT)
+    sort, _ = gpu_build.build_memory(log2, n, rt_log2_req=4)
+    gpu_build.set_tuning(0, 0, 50, 0)
+    budget = sort + outs + 8 * 256 if room == "scratch" else grid + outs // 2
+    assert sort + outs + 8 * 256 <= budget < grid + outs
+    a = _Arena(budget)
+    out = native.BuiltC()
+    vox = dev(pts)
+    native.check(native.lib().pyrb_build(ctypes.byref(a.ex), log2, 4, 0, 0, 0, vox.data_ptr(), n, ctypes.byref(out)))
+    assert a.refused > 0 and len(a.live) == 6
+    b = gpu_build.Built(out, None)
+    g = b.download()
+    assert_same_build(g, orc.gb_build(log2, 4, pts), label=room)
+    native.lib().pyrb_built_free(ctypes.byref(a.ex), ctypes.byref(out))
+    b._c = None
+    assert not a.live

@@ -4,6 +4,8 @@ GPU build at 130 bytes per voxel (tests/cpu_test.zig:1559-1629, measured with a
 counting Exec); the same cap holds here for the plain 256^3 noise build with its edit
 overlay and for the 1024^3 worst case, where the bounds, taken from the input size,
 are tight. The GPU suite checks that a real build reports the same bytes."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -42,3 +44,34 @@ def test_invalid_requests_are_rejected():
         gpu_build.build_memory(8, 1000, count=0)
     with pytest.raises(native.PyrbError):
         gpu_build.build_memory(0, 1000, chunk_log2=np.array([5, 2], np.uint32))
+
+
+# Sparse small volumes order their voxels in cells that the sort does without; an allocator
+# that cannot give those is asked for the sort's scratch. Refused altogether, a build with
+# many entries per cell, or one whose path is set, is not planned again.
+@pytest.mark.parametrize("entries,path,asked_again", [(1000, 0, True), (1000, 1, False), (1000, 2, False),
+                                                      (600_000, 0, False)])
+def test_refused_scratch_is_asked_for_without_the_cells(entries, path, asked_again):
+    asked = []
+
+    def refuse(_, n):
+        asked.append(int(n))
+        return 0
+
+    L = native.lib()
+    ex = native.Exec(alloc=native.ALLOC_FN(refuse), free=native.FREE_FN(lambda _, p: None))
+    out = native.BuiltC()
+    gpu_build.set_tuning(0, 0, 50, path)
+    try:
+        want = [gpu_build.build_memory(7, entries)[0]]
+        gpu_build.set_tuning(0, 0, 50, native.PATH_SORT)
+        if asked_again:
+            want.append(gpu_build.build_memory(7, entries)[0])
+            assert want[1] * 30 < want[0]
+        gpu_build.set_tuning(0, 0, 50, path)
+        # (the input is never read: nothing is launched without scratch)
+        assert L.pyrb_build(ctypes.byref(ex), 7, 3, 0, 0, 0, 256, entries, ctypes.byref(out)) == \
+            native.PYRB_ERROR_OUT_OF_MEMORY
+    finally:
+        gpu_build.set_tuning(0, 0, 50, 0)
+    assert asked == want and out.nodes == 0

@@ -93,3 +93,35 @@ def test_realtime_poisson_stream():
     s = srv.serve(reqs, realtime=True).summary()
     assert s["requests"] == 200 and s["p50_ms"] > 0 and s["p99_ms"] >= s["p50_ms"]
     srv.release_all()
+
+
+def test_sparse_chunks_are_served_within_the_budget_of_their_sort():
+    """128^3 chunks of 300 voxels: their cells take 17 MB, their sort a fraction of one."""
+    import torch
+    from pyrit_b200 import gpu_build, native
+    from pyrit_b200.serve import ChunkPool, ChunkServer
+    rng = np.random.default_rng(2)
+    K, n = 4, 300
+    vox = np.concatenate([rng.integers(0, 128, (K * n, 3)), rng.integers(1, 9, (K * n, 1))], 1).astype(np.uint32)
+    log2s = np.full(K, 7, np.uint32)
+    gpu_build.set_tuning(0, 0, 50, native.PATH_SORT)
+    sort, outs = gpu_build.build_memory(0, K * n + 64, chunk_log2=log2s, rt_log2_req=5)
+    gpu_build.set_tuning(0, 0, 50, 0)
+    grid, _ = gpu_build.build_memory(0, K * n + 64, chunk_log2=log2s, rt_log2_req=5)
+    budget = 2 * (sort + outs)
+    assert budget < grid // 4
+    pool = ChunkPool(dev(vox), np.arange(K + 1) * n, log2s)
+    reqs = _requests(pool, 12, seed=1)
+    for r in reqs:
+        r.edits = r.edits[:4]
+    srv = ChunkServer(pool, budget_bytes=budget, max_batch_voxels=K * n, max_inflight=1, rt_log2=5)
+    stats = srv.serve(reqs, realtime=False)
+    assert len(stats.latencies_ms) == len(reqs) and srv.arena.peak <= budget
+    last = max(r.rid for r in reqs)
+    res, host = srv.download(last)
+    r = srv.requests[last]
+    pts = np.concatenate([vox[r.chunk * n:(r.chunk + 1) * n], r.edits])
+    alone = gpu_build.build(7, 5, dev(pts), n_new=len(pts)).download()
+    assert np.array_equal(host.attrs[res.first_voxel:res.first_voxel + alone.voxel_count], alone.attrs)
+    srv.release_all()
+    torch.cuda.synchronize()
