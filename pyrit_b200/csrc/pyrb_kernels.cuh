@@ -2493,22 +2493,31 @@ __device__ __forceinline__ void pal_load(const uint32_t* attrs, uint32_t n, uint
 
 __global__ void __launch_bounds__(kBlock) k_pal_collect(PaletteDesc p) {
     grid_dep_wait();
-    __shared__ uint32_t s_val[kPalSlots], s_first[kPalSlots], s_found;
+    __shared__ uint32_t s_val[kPalSlots], s_first[kPalSlots], s_found, s_over;
     const uint32_t tile = blockIdx.x;
     if (threadIdx.x < kPalSlots) {
         s_val[threadIdx.x] = kPalEmpty;
         s_first[threadIdx.x] = 0xFFFFFFFFu;
     }
-    if (threadIdx.x == 0) s_found = 0;
     const uint32_t c = warp_upper_index(p.tile_of, p.count + 1, tile);
     if (c >= p.count) return;
     const uint32_t lo = __ldg(p.first + c) + (tile - __ldg(p.tile_of + c)) * kPalTile;
     const uint32_t hi = min(__ldg(p.first + c + 1), lo + kPalTile);
-    // (a chunk that another tile found to hold too many values: nothing more to learn)
-    if (*reinterpret_cast<volatile uint32_t*>(p.gflag + c) != 0) return;
+    // (a chunk that another tile found to hold too many values: nothing more to learn. Other
+    // blocks set the flag meanwhile: one thread's read decides for the block)
+    if (threadIdx.x == 0) {
+        s_found = 0;
+        s_over = *reinterpret_cast<volatile uint32_t*>(p.gflag + c);
+    }
+    __syncthreads();
+    if (s_over != 0) return;
+    // Whether the block has found more values than a palette holds (nothing more to learn).
+    // Other warps count on: one lane's read decides for the warp, which leaves as a whole.
+    auto full = [&]() -> bool {
+        return __shfl_sync(kFull, *reinterpret_cast<volatile uint32_t*>(&s_found), 0) > kPalMax;
+    };
     uint32_t v[kPalPer];
     pal_load(p.attrs + lo, hi - lo, v);
-    __syncthreads();
     // A thread passes over the two values it met last. Of the others in a row of the warp
     // each value is inserted once, by its lowest lane: a thread's rows and a row's lanes are
     // in index order, so the smallest index of a value is among the inserted ones.
@@ -2524,8 +2533,7 @@ __global__ void __launch_bounds__(kBlock) k_pal_collect(PaletteDesc p) {
             const bool need = x != kPalEmpty && x != last0 && x != last1;
             unsigned todo = __ballot_sync(kFull, need);
             if (!todo) continue;
-            // (more values than a palette holds: nothing more to learn)
-            if (*reinterpret_cast<volatile uint32_t*>(&s_found) > kPalMax) break;
+            if (full()) break;
             while (todo) {
                 const uint32_t lead = __ffs(todo) - 1;
                 todo &= ~__ballot_sync(kFull, x == __shfl_sync(kFull, x, lead));
@@ -2538,7 +2546,7 @@ __global__ void __launch_bounds__(kBlock) k_pal_collect(PaletteDesc p) {
                 last0 = x;
             }
         }
-        if (*reinterpret_cast<volatile uint32_t*>(&s_found) > kPalMax) break;
+        if (full()) break;
     }
     __syncthreads();
     if (s_found > kPalMax) {  // the chunk keeps its 32-bit attributes

@@ -127,3 +127,25 @@ def test_palette_steps_and_limits(size):
     first = np.arange(len(parts) + 1, dtype=np.uint32) * size
     attrs = np.concatenate(parts)
     _check_against_oracle(attrs, dev(attrs), first)
+
+
+# Chunks of many blocks whose warps find the values beyond a palette's 16 at about the same
+# time or one after another, beside chunks that just fit: the blocks' and warps' early ends.
+@pytest.mark.gpu
+@pytest.mark.parametrize("values", [17, 18, 64, 65, 5000])
+def test_palette_early_ends(values):
+    from gpu_helpers import dev
+    rng = np.random.default_rng(values)
+    parts = []
+    for size in (256, 5000, 16384, 200_000):
+        vals = rng.permutation(1 << 20)[:values].astype(np.uint32)
+        parts.append(rng.choice(vals, size))                          # everywhere at once
+        parts.append(np.sort(rng.choice(vals, size)))                 # in runs, warp after warp
+        one = np.full(size, vals[0], np.uint32)                       # in the last rows only
+        one[-min(values, size):] = vals[:min(values, size)]
+        parts.append(one)
+        parts.append(rng.choice(vals[:16], size))                     # a palette
+    first = np.concatenate([[0], np.cumsum([len(v) for v in parts])]).astype(np.uint32)
+    attrs = np.concatenate(parts).astype(np.uint32)
+    cnt = _check_against_oracle(attrs, dev(attrs), first)
+    assert (cnt == OVER).sum() >= 8 and (cnt[3::4] <= 16).all()
