@@ -1544,7 +1544,7 @@ PYRB_API pyrb_result pyrb_path_edit(const pyrb_exec* e, uint64_t nodes, uint64_t
     cudaStream_t st = e ? reinterpret_cast<cudaStream_t>(e->stream) : nullptr;
     Mem mem{e, st};
     const uint64_t edit_bytes = align_up(uint64_t(std::max(n_edits, 1u)) * 16, 256);
-    const uint64_t block = mem.get(align_up(plan.size(), 256) + 2 * edit_bytes);
+    const uint64_t block = mem.get(align_up(plan.size(), 256) + 2 * edit_bytes + uint64_t(count) * 4);
     if (!block) return fail(PYRB_ERROR_OUT_OF_MEMORY, "device memory for the path edits");
     PathEditDesc p;
     p.nodes = reinterpret_cast<uint32_t*>(nodes);
@@ -1556,6 +1556,7 @@ PYRB_API pyrb_result pyrb_path_edit(const pyrb_exec* e, uint64_t nodes, uint64_t
     uint4* given = reinterpret_cast<uint4*>(block + align_up(plan.size(), 256));
     p.given = given;
     p.edits = reinterpret_cast<uint4*>(reinterpret_cast<uint64_t>(given) + edit_bytes);
+    p.places = reinterpret_cast<uint32_t*>(reinterpret_cast<uint64_t>(given) + 2 * edit_bytes);
     p.count = count;
     auto done = [&](pyrb_result r) {
         if (r != PYRB_OK) cudaStreamSynchronize(st);  // the caller's arrays may still be read

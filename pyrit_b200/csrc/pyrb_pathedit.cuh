@@ -64,6 +64,7 @@ struct PathEditDesc {
                                  // attribute map (what, place, value, 0)
     const uint32_t* attr_tile;   // [count + 1] first attribute tile of each job
     const uint32_t* prim_tile;   // [count + 1] first prim tile of each job
+    uint32_t* places;            // [count] attributes of the job's target that come from its source or an operation
     uint32_t count;
 };
 
@@ -291,6 +292,7 @@ __global__ void __launch_bounds__(32) k_path_walk(PathEditDesc p) {
     }
     __syncwarp();
     uint32_t root = job.root, flags = 0, count = job.attr_count;
+    int32_t undone = 0;  // voxels that a brick gained whose path found no room
     uint32_t e = 0;
     while (e < n_edits) {
         const uint4 lead = edits[e];
@@ -351,6 +353,7 @@ __global__ void __launch_bounds__(32) k_path_walk(PathEditDesc p) {
             uint32_t nr = 0, sub = 0;
             if (!pe_rewrite(w, s_path, wk, job.log2_size, job.rt_log2, v0, brick, delta, &has_root, &nr, &has_sub, &sub)) {
                 flags |= kPeOverflow;
+                undone = delta;
                 continue;
             }
             if (has_root) root = nr; else flags |= kPeEmpty;
@@ -368,6 +371,12 @@ __global__ void __launch_bounds__(32) k_path_walk(PathEditDesc p) {
         out.out_count = count;
         out.out_attr_b = 0;
         out.out_flags = flags;
+        // The operations of a brick whose path found no room stay in the list, but the tree
+        // and the count are those before it. With more removals than inserts among them the
+        // list is shorter than the count: the places behind it have no source (they would come
+        // from behind the job's attributes), and the map makes them 0. (The result of such a
+        // job is not used.)
+        p.places[j] = flags & kPeEmpty ? 0u : undone < 0 ? count - uint32_t(-undone) : count;
     }
 }
 
@@ -429,6 +438,11 @@ __global__ void __launch_bounds__(kBlock) k_path_map(PathEditDesc p) {
         ops[k].x = what;
         ops[k].y = place;
     }
+    if (job.out_flags & kPeEmpty) return;
+    // (the word of the last place that has a source is the rewrite's)
+    const uint32_t per = job.palette ? 8 : 1, end = (job.out_count + per - 1) / per;
+    uint32_t* dst = p.attrs + job.attr_a;
+    for (uint32_t i = (p.places[blockIdx.x] + per - 1) / per + threadIdx.x; i < end; i += kBlock) dst[i] = 0;
 }
 
 // 3. Attributes of every job, kPeTile outputs per CTA in kPeSteps steps (pathedit.zig:
@@ -447,9 +461,9 @@ __global__ void __launch_bounds__(kBlock) k_path_attrs(PathEditDesc p) {
     const uint32_t j = warp_upper_index(p.attr_tile, p.count + 1, tile);
     if (j >= p.count) return;
     const PathEditJob& job = p.jobs[j];
-    const uint32_t n_ops = min(job.edit_count, kPeMaxEdits), n_final = job.out_count;
+    const uint32_t n_ops = min(job.edit_count, kPeMaxEdits), n_final = p.places[j];
     const uint32_t tile0 = (tile - __ldg(p.attr_tile + j)) * kPeTile;
-    if ((job.out_flags & kPeEmpty) || tile0 >= n_final) return;
+    if (tile0 >= n_final) return;
     const uint4* ops = p.edits + job.edit_first;
     {
         uint32_t before[kPeSteps] = {}, inside = 0;  // (differences: may wrap)

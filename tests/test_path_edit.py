@@ -263,3 +263,50 @@ def test_cuda_path_edit_tiles_and_repeats(log2, rt, n_edits, kind):
     assert np.array_equal(da.cpu().numpy().view(np.uint32), a2)
     assert np.array_equal(dp.cpu().numpy().reshape(-1), p2.reshape(-1))
     assert np.array_equal(db.cpu().numpy().reshape(-1).view(np.uint32), b2.reshape(-1).view(np.uint32))
+
+
+# A job whose arena has no room for the path of a brick that loses all its voxels: its count
+# stays, its operations are there, and the last places of its target would come from behind
+# its attributes. Here nothing of the caller's lies there: the source ends the pool, and
+# words of a later owner follow it.
+@pytest.mark.gpu
+@pytest.mark.parametrize("palette", [False, True])
+@pytest.mark.parametrize("room", [4, 12])
+def test_cuda_path_edit_overflow_reads_its_own_attributes_only(palette, room):
+    from pyrit_b200 import gpu_build, native
+    from gpu_helpers import dev
+    log2, rt = 5, 4
+    brick = np.array([[x, y, z, 1 + (x + y + z) % 5] for z in range(4) for y in range(4) for x in range(4)], np.uint32)
+    vox = np.concatenate([brick, brick + np.array([8, 8, 8, 0], np.uint32)])
+    g = orc.gb_build(log2, rt, vox)
+    ed = brick + np.array([8, 8, 8, 0], np.uint32)
+    ed[:, 3] = 0
+    if room > 4:  # room for the path of an earlier brick
+        ed = np.concatenate([np.array([[4, 0, 0, 3]], np.uint32), ed])
+    job = _job(g, log2, rt, len(ed), node_cap=room)
+    cap = job["attr_cap"]
+    src, first = g.attrs, np.array([0, g.voxel_count], np.uint32)
+    job.update(attr_a=0, attr_src=cap)
+    if palette:
+        pal, counts = orc.palette_scan(g.attrs, first)
+        dst, total = orc.palette_layout(first, counts)
+        src = orc.palette_pack(g.attrs, first, pal, counts, dst, total)
+        job.update(palette=1, pal_src=cap + 16, attr_src=cap + 32, pal_dst=0, attr_a=16, attr_cap=cap - 16)
+        src = np.concatenate([np.zeros(16, np.uint32), src])
+    pool = np.concatenate([np.zeros(cap, np.uint32), src])
+    behind = np.full(128, 0x77777777, np.uint32)
+    nodes = np.concatenate([g.nodes, np.zeros(room, np.uint32)])
+    leaves = np.concatenate([g.leaves, np.zeros(job["leaf_cap"], np.uint64)])
+    n2, l2, a2, p2, b2, want = orc.path_edit(nodes, leaves, np.concatenate([pool, 0 * behind]), [job], ed, g.prims, g.aabbs)
+    assert want[0]["out_flags"] & OVERFLOW and want[0]["out_count"] == g.voxel_count + (room > 4)
+    dn, dl, da = dev(nodes), dev(leaves), dev(np.concatenate([pool, behind]))
+    dp, db = dev(g.prims), dev(g.aabbs.view(np.uint32))
+    j = native.PathEditJob(**job)
+    j.prims, j.aabbs = dp.data_ptr(), db.data_ptr()
+    out = [j]
+    gpu_build.path_edit(dn, dl, da, out, ed)
+    assert (out[0].out_root, out[0].out_count, out[0].out_flags) == tuple(
+        want[0][k] for k in ("out_root", "out_count", "out_flags"))
+    assert np.array_equal(dn.cpu().numpy().view(np.uint32), n2)
+    got = da.cpu().numpy().view(np.uint32)
+    assert np.array_equal(got[:len(pool)], a2[:len(pool)]) and np.array_equal(got[len(pool):], behind)
