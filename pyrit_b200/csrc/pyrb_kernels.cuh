@@ -2502,7 +2502,8 @@ __global__ void __launch_bounds__(kBlock) k_pal_collect(PaletteDesc p) {
     const uint32_t c = warp_upper_index(p.tile_of, p.count + 1, tile);
     if (c >= p.count) return;
     const uint32_t lo = __ldg(p.first + c) + (tile - __ldg(p.tile_of + c)) * kPalTile;
-    const uint32_t hi = min(__ldg(p.first + c + 1), lo + kPalTile);
+    // (differences: the tile's end may lie beyond 32 bits)
+    const uint32_t hi = lo + min(__ldg(p.first + c + 1) - lo, kPalTile);
     // (a chunk that another tile found to hold too many values: nothing more to learn. Other
     // blocks set the flag meanwhile: one thread's read decides for the block)
     if (threadIdx.x == 0) {
@@ -2525,7 +2526,7 @@ __global__ void __launch_bounds__(kBlock) k_pal_collect(PaletteDesc p) {
     // reference.)
     const unsigned lane = threadIdx.x & 31;
     uint32_t last0 = kPalEmpty, last1 = kPalEmpty;
-    for (uint32_t base = lo; base < hi; base += kPalStep) {
+    for (uint32_t base = lo; base - lo < hi - lo; base += kPalStep) {
         if (base != lo) pal_load(p.attrs + base, hi - base, v);
 #pragma unroll
         for (uint32_t k = 0; k < kPalPer; ++k) {
@@ -2622,17 +2623,17 @@ __global__ void __launch_bounds__(kBlock) k_pal_pack(PaletteDesc p) {
     if (c >= p.count) return;
     const uint32_t lo = __ldg(p.first + c), n = __ldg(p.first + c + 1) - lo;
     const uint32_t t0 = (tile - __ldg(p.tile_of + c)) * kPalTile;  // first voxel of the tile within the chunk
-    const uint32_t t1 = min(n, t0 + kPalTile);
+    const uint32_t t1 = t0 + min(n - t0, kPalTile);
     uint32_t* out = p.pool + __ldg(p.dst + c);
     const bool raw = __ldg(p.counts + c) == kPalOverflow;
     uint32_t v[kPalPer];
     pal_load(p.attrs + lo + t0, t1 - t0, v);
     if (raw) {
-        for (uint32_t base = t0; base < t1; base += kPalStep) {
+        for (uint32_t base = t0; base - t0 < t1 - t0; base += kPalStep) {
             if (base != t0) pal_load(p.attrs + lo + base, t1 - base, v);
 #pragma unroll
             for (uint32_t k = 0; k < kPalPer; ++k)
-                if (base + k * kBlock + threadIdx.x < t1) out[base + k * kBlock + threadIdx.x] = v[k];
+                if (k * kBlock + threadIdx.x < t1 - base) out[base + k * kBlock + threadIdx.x] = v[k];
         }
         return;
     }
@@ -2654,7 +2655,7 @@ __global__ void __launch_bounds__(kBlock) k_pal_pack(PaletteDesc p) {
     __syncthreads();
     const uint32_t none = s_none < kPalMax ? s_none : 0u;
     uint32_t last = kPalEmpty, ix = none;
-    for (uint32_t base = t0; base < t1; base += kPalStep) {
+    for (uint32_t base = t0; base - t0 < t1 - t0; base += kPalStep) {
         if (base != t0) pal_load(p.attrs + lo + base, t1 - base, v);
 #pragma unroll
         for (uint32_t k = 0; k < kPalPer; ++k) {
@@ -2667,11 +2668,12 @@ __global__ void __launch_bounds__(kBlock) k_pal_pack(PaletteDesc p) {
                 for (uint32_t key; last != kPalEmpty && (key = s_val[s]) != kPalEmpty; s = (s + 1) & (kPalSlots - 1))
                     if (key == last) { ix = s_ix[s]; break; }
             }
-            uint32_t word = i < t1 ? ix << ((threadIdx.x & 7) * 4) : 0u;
+            const bool in = k * kBlock + threadIdx.x < t1 - base;
+            uint32_t word = in ? ix << ((threadIdx.x & 7) * 4) : 0u;
             word |= __shfl_xor_sync(kFull, word, 1);
             word |= __shfl_xor_sync(kFull, word, 2);
             word |= __shfl_xor_sync(kFull, word, 4);
-            if ((threadIdx.x & 7) == 0 && i < t1) out[kPalMax + i / 8] = word;
+            if ((threadIdx.x & 7) == 0 && in) out[kPalMax + i / 8] = word;
         }
     }
 }

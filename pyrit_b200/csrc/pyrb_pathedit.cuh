@@ -494,8 +494,8 @@ __global__ void __launch_bounds__(kBlock) k_path_attrs(PathEditDesc p) {
     const uint32_t* src = p.attrs + job.attr_src;
     uint32_t* dst = p.attrs + job.attr_a;
     for (uint32_t s = 0; s < kPeSteps; ++s) {
-        const uint32_t t0 = tile0 + s * kPeStep, t1 = min(t0 + kPeStep, n_final);
-        if (t0 >= n_final) break;
+        if (n_final - tile0 <= s * kPeStep) break;  // (differences: a step's end may lie beyond 32 bits)
+        const uint32_t t0 = tile0 + s * kPeStep, m = min(n_final - t0, kPeStep);
         const bool inside = (in_steps >> s) & 1;
         uint32_t dist0 = 0;
 #pragma unroll
@@ -528,8 +528,8 @@ __global__ void __launch_bounds__(kBlock) k_path_attrs(PathEditDesc p) {
             __syncthreads();
         }
         if (job.palette) {
-            for (uint32_t wd = t0 / 8 + threadIdx.x; wd < (t1 + 7) / 8; wd += kBlock) {
-                const uint32_t i0 = wd * 8, n = min(t1 - i0, 8u);
+            for (uint32_t wd = t0 / 8 + threadIdx.x; wd < t0 / 8 + (m + 7) / 8; wd += kBlock) {
+                const uint32_t i0 = wd * 8, n = min(n_final - i0, 8u);
                 uint32_t word = 0;
                 if (!inside) {
                     const uint32_t a = i0 + dist0, b = a + n - 1;
@@ -554,13 +554,13 @@ __global__ void __launch_bounds__(kBlock) k_path_attrs(PathEditDesc p) {
         for (uint32_t k = 0; k < kPer; ++k) {
             const uint32_t i = threadIdx.x + k * kBlock;
             v[k] = 0;
-            if (t0 + i >= t1) continue;
+            if (i >= m) continue;
             const uint32_t took = inside ? s_took[i] : 0u;
             v[k] = took ? ops[took - 1].z : src[t0 + i + (inside ? uint32_t(s_dist[i]) : dist0)];
         }
 #pragma unroll
         for (uint32_t k = 0; k < kPer; ++k)
-            if (t0 + threadIdx.x + k * kBlock < t1) dst[t0 + threadIdx.x + k * kBlock] = v[k];
+            if (threadIdx.x + k * kBlock < m) dst[t0 + threadIdx.x + k * kBlock] = v[k];
     }
 }
 

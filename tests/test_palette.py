@@ -149,3 +149,33 @@ def test_palette_early_ends(values):
     attrs = np.concatenate(parts).astype(np.uint32)
     cnt = _check_against_oracle(attrs, dev(attrs), first)
     assert (cnt == OVER).sum() >= 8 and (cnt[3::4] <= 16).all()
+
+
+# Chunks whose voxels have the last indices of 32 bits: a block of 16384 voxels that starts
+# there would end beyond them. The buffer holds these chunks only (an address that far below
+# it stands for the attributes before them, which nothing reads).
+@pytest.mark.gpu
+@pytest.mark.parametrize("sizes", [(1,), (16383,), (16384,), (16385, 4095), (3, 40000, 5000)])
+def test_palette_of_the_last_voxel_indices(sizes):
+    import torch
+    from pyrit_b200 import gpu_build
+    from gpu_helpers import dev
+    rng = np.random.default_rng(len(sizes))
+    n = sum(sizes)
+    attrs = np.concatenate([rng.integers(0, 5 if c % 2 else 17, k) for c, k in enumerate(sizes)]).astype(np.uint32)
+    ofirst = np.concatenate([[0], np.cumsum(sizes)]).astype(np.uint32)
+    base = 0xFFFFFFFF - n
+    first = (ofirst.astype(np.int64) + base).astype(np.uint32)
+    assert first[-1] == 0xFFFFFFFF
+    buf = dev(attrs)
+    addr = buf.data_ptr() - 4 * base
+    pal, cnt = gpu_build.palette_scan(addr, first)
+    opal, ocnt = orc.palette_scan(attrs, ofirst)
+    assert np.array_equal(cnt, ocnt)
+    keep = ocnt != OVER
+    assert np.array_equal(pal.cpu().numpy().view(np.uint32)[keep], opal[keep])
+    dst, total = orc.palette_layout(ofirst, ocnt)
+    pool = torch.zeros(max(total, 1), dtype=torch.int32, device="cuda")
+    gpu_build.palette_pack(addr, first, pal, cnt, dst, pool)
+    opool = orc.palette_pack(attrs, ofirst, opal, ocnt, dst, total)
+    assert np.array_equal(pool.cpu().numpy().view(np.uint32)[:total], opool)
