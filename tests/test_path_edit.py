@@ -222,8 +222,9 @@ def _decode(keys):
     return out
 
 
-# The attribute rewrite takes tiles of 4096 attributes and traces every operation once:
-# operations at the tiles' first and last places, voxels set, removed and set again in one
+# The attribute rewrite takes steps of 4096 attributes in tiles of 16384 and traces every
+# operation once:
+# operations at the steps' first and last places, voxels set, removed and set again in one
 # job, the most edits a job takes, more prims than the walk keeps in shared memory, and
 # one prim over the whole volume.
 @pytest.mark.gpu
@@ -310,3 +311,71 @@ def test_cuda_path_edit_overflow_reads_its_own_attributes_only(palette, room):
     assert np.array_equal(dn.cpu().numpy().view(np.uint32), n2)
     got = da.cpu().numpy().view(np.uint32)
     assert np.array_equal(got[:len(pool)], a2[:len(pool)]) and np.array_equal(got[len(pool):], behind)
+
+
+def _edited_by_both(job, nodes, leaves, attrs, ed, prims, aabbs):
+    """The CUDA path edit against the oracle's, byte for byte; returns the oracle's boxes."""
+    from pyrit_b200 import gpu_build, native
+    from gpu_helpers import dev
+    nodes = np.concatenate([nodes, np.zeros(job["node_cap"], np.uint32)])
+    leaves = np.concatenate([leaves, np.zeros(job["leaf_cap"], np.uint64)])
+    attrs = np.concatenate([attrs, np.zeros(job["attr_cap"], np.uint32)])
+    n2, l2, a2, p2, b2, want = orc.path_edit(nodes, leaves, attrs, [job], ed, prims, aabbs)
+    dn, dl, da, dp, db = dev(nodes), dev(leaves), dev(attrs), dev(prims), dev(aabbs.view(np.uint32))
+    j = native.PathEditJob(**job)
+    j.prims, j.aabbs = dp.data_ptr(), db.data_ptr()
+    out = [j]
+    gpu_build.path_edit(dn, dl, da, out, ed)
+    assert (out[0].out_root, out[0].out_count, out[0].out_flags) == tuple(
+        want[0][k] for k in ("out_root", "out_count", "out_flags"))
+    assert np.array_equal(dn.cpu().numpy().view(np.uint32), n2)
+    assert np.array_equal(dl.cpu().numpy().view(np.uint64), l2)
+    assert np.array_equal(da.cpu().numpy().view(np.uint32), a2)
+    assert np.array_equal(dp.cpu().numpy().reshape(-1), p2.reshape(-1))
+    assert np.array_equal(db.cpu().numpy().reshape(-1).view(np.uint32), b2.reshape(-1).view(np.uint32))
+    return b2
+
+
+# Boxes of subtrees up to 2^10, by a warp with a stack in shared memory, and beyond, by one
+# lane: the edges around the limit, few voxels in each prim and many.
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [30, 20000])
+@pytest.mark.parametrize("log2,rt", [(7, 7), (9, 8), (10, 9), (10, 10), (11, 10), (11, 11), (12, 11)])
+def test_cuda_path_edit_boxes_of_large_subtrees(log2, rt, n):
+    rng = np.random.default_rng(log2 * 100 + rt + n)
+    vox = np.concatenate([rng.integers(0, 1 << log2, (n, 3)), rng.integers(1, 9, (n, 1))], 1).astype(np.uint32)
+    g = orc.gb_build(log2, rt, vox)
+    ed = _edits(rng, log2, vox, 40)
+    _edited_by_both(_job(g, log2, rt, len(ed)), g.nodes, g.leaves, g.attrs, ed, g.prims, g.aabbs)
+
+
+# Full and nearly full trees of a 2^10 prim (8^8 bricks on a handful of shared nodes): the
+# stack of the warp's walk at its deepest.
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", ["full", "shared"])
+def test_cuda_path_edit_box_of_a_full_subtree(kind):
+    rng = np.random.default_rng(5)
+    log2 = rt = 10
+    leaf = np.array([1 << 21, 1 << 42, (1 << 21) | (1 << 22)], np.uint64)  # inner cells of a brick only
+    count = [1, 1, 2]
+    below = [(k, count[k]) for k in range(1 if kind == "full" else 3)]     # (reference, voxels) one level down
+    nodes = []
+    for s in range(2, log2):
+        here = []
+        for _ in range(1 if kind == "full" or s == log2 - 1 else 3):
+            # (the first and last child stay: the whole cube is to be looked at)
+            mask = 0xFF if kind == "full" or s == log2 - 1 else 0x81 | int(rng.integers(0, 256)) | 0x18
+            kids = [below[int(rng.integers(len(below)))] for k in range(8) if mask >> k & 1]
+            here.append((len(nodes), sum(c for _, c in kids)))
+            nodes += [mask, sum(c for _, c in kids)] + [r for r, _ in kids]
+        below = here
+    root, voxels = below[0]
+    attrs = (1 + np.arange(voxels) % 200).astype(np.uint32)
+    ed = np.array([[1, 1, 1, 9], [2, 1, 1, 9], [1021, 1020, 1022, 9]], np.uint32)
+    job = dict(node_offset=0, leaf_offset=0, root=root, log2_size=log2, attr_src=0, attr_count=voxels, attr_a=voxels,
+               attr_b=0, attr_cap=voxels + 3, palette=0, pal_src=0, pal_dst=0, node_arena=len(nodes), node_cap=400,
+               leaf_arena=len(leaf), leaf_cap=3, edit_first=0, edit_count=3, rt_log2=rt, prim_count=1, aabbs_keep=0)
+    prim = np.zeros(16, np.uint8)
+    prim[:4] = np.frombuffer(np.uint32(root).tobytes(), np.uint8)
+    box = _edited_by_both(job, np.array(nodes, np.uint32), leaf, attrs, ed, prim, np.zeros(6, np.float32))
+    assert (box.reshape(-1)[3:] - box.reshape(-1)[:3] > 1000).all()
