@@ -99,21 +99,22 @@ __device__ __forceinline__ void for_tile_entries(const BuildDesc& d, const TileS
     const uint32_t j0 = sp.start - seg_begin - (d.one_seg ? d.n_old : 0u);
     if (d.mode == kModeDownsample) {
         const unsigned lane = threadIdx.x & 31;
+        const uint64_t outside = ~((d.grid_cells << (3 * d.shift)) - 1);  // bits of keys outside the source volume
         for (uint32_t base = 0; base < sp.count; base += kScatterBatch * kBlock) {
             uint64_t src[kScatterBatch];
             uint32_t val[kScatterBatch];
 #pragma unroll
             for (int k = 0; k < kScatterBatch; ++k) {
                 const uint32_t idx = base + k * kBlock + threadIdx.x;
-                src[k] = idx < sp.count ? __ldcs(d.src_keys + sp.start + idx) : 0;
+                src[k] = idx < sp.count ? __ldcs(d.src_keys + sp.start + idx) : ~0ull;
                 val[k] = idx < sp.count ? __ldcs(d.src_vals + sp.start + idx) : 0u;
             }
 #pragma unroll
             for (int k = 0; k < kScatterBatch; ++k) {
                 const uint32_t idx = base + k * kBlock + threadIdx.x;
-                // (a source key outside the volume has no cell: compared before it is cut to 32 bits)
-                const uint64_t coarse = coarse_key(src[k], d.shift);
-                const uint32_t key = idx < sp.count && coarse < d.grid_cells ? uint32_t(coarse) : 0xFFFFFFFFu;
+                // (a source key outside the volume has no cell)
+                const bool out = (src[k] & outside) != 0;
+                const uint32_t key = out ? 0xFFFFFFFFu : uint32_t(coarse_key(src[k], d.shift));
                 // the source voxels come in key order (x + 4y + 16z inside a brick): up to 8
                 // of them share a coarse cell, at distances 1, 4 and 16 in full bricks. Of a
                 // row's entries of a cell only the last can decide: those that a later one of
@@ -121,7 +122,7 @@ __device__ __forceinline__ void for_tile_entries(const BuildDesc& d, const TileS
                 const uint32_t n1 = __shfl_down_sync(kFull, key, 1), n4 = __shfl_down_sync(kFull, key, 4),
                                n16 = __shfl_down_sync(kFull, key, 16);
                 const bool later = (lane < 31 && n1 == key) || (lane < 28 && n4 == key) || (lane < 16 && n16 == key);
-                if (key != 0xFFFFFFFFu && !later) f(sp.start + idx, key, val[k]);
+                if (!out && !later) f(sp.start + idx, key, val[k]);
             }
         }
         return;
