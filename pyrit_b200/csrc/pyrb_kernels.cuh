@@ -1749,7 +1749,9 @@ __device__ __forceinline__ void node_own_tile(const BuildDesc& d, const LevelDes
 }
 
 // Fewer blocks than there may be tiles: they take tile after tile (4096^3 surface, levels 2
-// to 5: 25 + 18 + 18 + 14 -> 20 + 14 + 14 + 13 us; 1024^3 level 2: 154 -> 144).
+// to 5: 25 + 18 + 18 + 14 -> 20 + 14 + 14 + 13 us; 1024^3 level 2: 154 -> 144). A level
+// without parents has no tile and writes no cursor for the next: then every level is empty,
+// and all cursors stay 0.
 template <int NIT>
 __global__ void __launch_bounds__(kBlock) k_node_own(BuildDesc d, LevelDesc L) {
     grid_dep_wait();
@@ -1764,12 +1766,6 @@ __global__ void __launch_bounds__(kBlock) k_node_own(BuildDesc d, LevelDesc L) {
         node_own_tile<NIT>(d, L, tile, P, cursor);
         if (ntiles <= gridDim.x) return;
     }
-}
-
-// Empty levels still have to pass the cursor on.
-__global__ void k_level_cursor(BuildDesc d, uint32_t lv) {
-    grid_dep_wait();
-    if (threadIdx.x == 0 && d.counters[kCtrParents + lv] == 0) d.counters[kCtrCursor + lv + 1] = d.counters[kCtrCursor + lv];
 }
 
 // ---------------------------------------------------------------------------
