@@ -78,9 +78,13 @@ std::atomic<uint32_t> g_path{kPathAuto};
 // The grid path is taken automatically while the chunks hold at most 4 cells per entry
 // (dense volumes: 256^3 noise at 30 % solid has 3.3, terrain chunks 2) or 2^23 cells more
 // than that, and at most kGridMaxCells cells in all (8 B each). The bytes of a grid of 2^23
-// cells stay in the L2, and the sort's passes have a floor of some 80 us however few the
+// cells stay in the L2, and the sort's passes have a floor of their own however few the
 // entries are: a 128^3 scene of 295,000 voxels (7 cells per entry) orders in 35 us on the
-// grid, 92 sorted; beyond both terms the cells' traffic loses (1024^3 at 15 %, 6.6 cells
+// grid, 92 sorted. Whole calls, grid and sort: 128^3 with 10 / 1000 / 30,000 / 300,000 entries
+// 65 / 67 / 114 / 125 and 75 / 92 / 158 / 158 us; 4 chunks of 128^3 (all 2^23 cells) with
+// 400 / 4000 / 40,000 entries 166 / 234 / 228 and 158 / 229 / 247, 256 of 32^3 with 25,600
+// 218 and 207: at the full 2^23 the sort of a hundred entries a chunk is up to 10 us
+// shorter. Beyond both terms the cells' traffic loses (1024^3 at 15 %, 6.6 cells
 // per entry: 9.3 ms against 5.3).
 constexpr uint64_t kGridCellsPerEntry = 4, kGridFreeCells = uint64_t(1) << 23;
 // A node level takes tiles of one item per thread below this many large tiles (2 per SM)
@@ -517,6 +521,10 @@ pyrb_result plan_build(const Job& job, const Tune* fixed, Plan& p, bool lean = f
         if (rb == 0) {
             auto_tuning(lb - 6, &rb, &tile_keys);
             // chunks that a 4096-entry tile (nearly) holds would leave 8192-entry ones half empty
+            // (entries on average, capacities where the counts are on the device). 9-bit digits,
+            // tiles of 4096 and 8192, us a call: 1063 chunks of 32^3 with 500 / 3000 / 6000
+            // entries 331 / 389 / 484 and 354 / 432 / 475, with every other chunk nearly empty
+            // 406 (3000) / 466 (6000) and 428 / 521; 64 of 256^3 with 6000 429 and 441
             if (K > 1 && nmax <= uint64_t(K) * 6144) tile_keys = 4096;
         }
         lf = g_load_pct.load();

@@ -42,12 +42,8 @@ __device__ __forceinline__ void red_max_u64(uint64_t* p, uint64_t v) {
     asm volatile("red.relaxed.gpu.global.max.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
 
-// Every entry of a tile with a valid key, in the per-segment tiling of the sort path
-// (tile_span), so the entry index (the order that decides) and the chunk are those of
-// the sort: f(entry index, local key, value). PyrVoxel segments (every mode but old
-// keys and downsampling) take the fast loop: the chunk's voxel and edit lists are
-// resolved once per tile, and each thread keeps kScatterBatch 16-byte loads in flight
-// before it encodes them.
+// The entries of a tile: the per-segment tiling of the sort path (tile_span), so that the
+// entry index (the order that decides) and the chunk are those of the sort.
 // A single volume is one stretch of entries: no plan to look anything up in.
 __device__ __forceinline__ TileSpan grid_span(const BuildDesc& d, uint32_t tile) {
     if (!d.one_seg) return tile_span(d, tile);
@@ -59,6 +55,11 @@ __device__ __forceinline__ TileSpan grid_span(const BuildDesc& d, uint32_t tile)
     return t;
 }
 
+// Every entry of a tile with a valid key: f(entry index, local key, value). PyrVoxel
+// segments take the last loop: the chunk's voxel and edit lists are resolved once per tile,
+// and each thread keeps kScatterBatch 16-byte loads in flight before it encodes them. The
+// source keys of a downsample have a loop of their own; old keys on the buckets take the
+// general one (on the grid k_grid_old stores them).
 constexpr int kScatterBatch = 4;
 template <typename F>
 __device__ __forceinline__ void for_tile_entries(const BuildDesc& d, const TileSpan& sp, F&& f) {

@@ -1,6 +1,8 @@
-// Kernels of the DAG build (sm_100a). One build = plan -> encode/histogram ->
-// onesweep radix passes -> unique -> bricks (+ leaf insert) -> leaf owners ->
-// per level {node build (+ insert), node owners} -> prims -> finalize.
+// Kernels of the DAG build (sm_100a). One build = plan -> encode/histogram -> digit
+// bases -> onesweep radix passes -> unique voxels and bricks (or the cell grid or the
+// brick buckets instead) -> leaf inserts -> leaf owners -> per level {node build, node
+// inserts, node owners}, prims after their level -> tail: the levels of few children,
+// the leaves of small builds, roots and final counts.
 //
 // Every kernel that assigns output positions uses a decoupled look-back over
 // dynamically numbered tiles: a tile only ever waits for tiles with smaller
@@ -75,8 +77,6 @@ __device__ __forceinline__ uint32_t dyn_tile_and(uint32_t* counters, uint32_t ct
     return t;
 }
 
-// 6 tiles per SM for the small levels; large tiles keep their parent's references in
-// registers and take 5 (51 registers, no spills)
 // ---------------------------------------------------------------------------
 // Segment plan: first entry and first sort tile of every segment.
 // ---------------------------------------------------------------------------
@@ -1568,6 +1568,8 @@ __device__ __forceinline__ void node_build_tile(const BuildDesc& d, const LevelD
     }
 }
 
+// 6 tiles per SM for the small levels; large tiles keep their parent's references in
+// registers and take 5 (48 registers)
 template <int NB>
 __global__ void __launch_bounds__(kBlock, NB == 1 ? 6 : 5) k_node_build(BuildDesc d, LevelDesc L) {
     grid_dep_wait();
@@ -1813,18 +1815,19 @@ __global__ void __launch_bounds__(kBlock) k_prims(BuildDesc d, LevelDesc L) {
 }
 
 // ---------------------------------------------------------------------------
-// Upper levels in one CTA. Each level: stage the children in shared memory, find
-// heads (block scan), build the parents' words into global memory (their hashes into
-// shared memory), dedup them in a shared-memory table (owner = minimum parent index),
+// Upper levels in one CTA, and the leaves of builds whose bricks are few enough. Each
+// level: stage the children in shared memory, find heads (block scan), build the
+// parents' words, dedup them in a shared-memory table (owner = minimum parent index),
 // give the owners word offsets (block scan of their lengths), write their words, and
 // turn every parent's slot into its node offset, which the next level uses as the
 // child reference. Prims (level rt_log2 - 1), roots and the final counts are written
-// here as well. Same output as k_node_build/k_node_own/k_prims/k_finalize per level.
+// here as well. Same output as k_node_build/k_node_insert/k_node_own/k_prims per level.
 // A global round trip costs about a microsecond here and a level has only a few
 // thousand parents, so the kernel is latency-bound: every load of a step is issued
-// before the first is used (loops unrolled over the thread's fixed share), children
-// and their boxes are staged in shared memory, and words are read back from global
-// memory only to compare two parents with equal hashes and to copy the owners out.
+// before the first is used (loops unrolled over the thread's fixed share), and children
+// and their boxes are staged in shared memory. The records and words of a level of more
+// than kTailSmall parents go to global memory (their hashes to shared memory) and are read
+// back only to compare two parents with equal hashes and to copy the owners out.
 // ---------------------------------------------------------------------------
 constexpr uint32_t kTailPer = kTailMaxChildren / kTailThreads;  // children (and parents) per thread
 constexpr uint32_t kTailScanWords = 72;
