@@ -94,6 +94,10 @@ constexpr uint32_t kSmallLevelTiles = 296;
 // cost the encode 0 to 4 us, which is what they save below some 2 M (1.3 M: 23.0 -> 22.9, encode
 // 21.5 -> 25.5)
 constexpr uint64_t kLargeTiles64 = uint64_t(1) << 21;
+// Chunks of a mixed batch up to which the tail's one block finds the roots of those smaller
+// than the batch's edge. Its 1024 threads take 2 / 6 / 22 / 92 us for 2000 / 8192 / 32,768 /
+// 100,000 chunks, the kernel for it 7
+constexpr uint32_t kTailChunks = 8192;
 // Blocks of the kernels that take tile after tile where the bounds ask for more: 8 per SM
 constexpr uint32_t kTileBlocks = 148u * 8u;
 constexpr uint64_t kGridMaxCells = uint64_t(1) << 33;
@@ -913,8 +917,9 @@ uint32_t launch_plan(const Plan& p, const std::vector<LevelDesc>& levels, cudaSt
         launches += 2;
     }
     const bool down = d.mode == kModeBatch && p.min_log2 < d.log2;
-    launches += launch_levels(d, levels, lv0, make_tail(lv0, p.P, levels, down), st, prof);
-    if (down && lv0 == d.log2) {  // no tail
+    const bool down_in_tail = down && lv0 < d.log2 && p.K <= kTailChunks;
+    launches += launch_levels(d, levels, lv0, make_tail(lv0, p.P, levels, down_in_tail), st, prof);
+    if (down && !down_in_tail) {
         launch(k_batch_roots, std::max(std::min((p.K + 255) / 256, 1024u), 1u), 256, 0, st, d);
         prof.mark("batch_roots");
         ++launches;

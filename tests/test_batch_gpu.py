@@ -129,3 +129,19 @@ def test_config2_mix_at_full_chunk_sizes(with_edits, path):
         _check(log2s, chunks, edits, rt=5)
     finally:
         gpu_build.set_tuning(0, 0, 50, native.PATH_AUTO)
+
+
+@pytest.mark.parametrize("K", [8192, 8193])
+def test_many_nearly_empty_chunks(K):
+    """The roots of the smaller chunks found by the tail's block, or by a kernel of their own
+    where the batch has more chunks."""
+    rng = np.random.default_rng(K)
+    log2s = rng.integers(3, 5, K)
+    log2s[0], log2s[-1] = 4, 3
+    held = np.concatenate([[0, K - 1], rng.choice(K, 300, replace=False)])
+    chunks = [np.zeros((0, 4), np.uint32)] * K
+    for c in held:
+        pts = rng.integers(0, 1 << log2s[c], (5, 4)).astype(np.uint32)
+        pts[:, 3] += 1
+        chunks[c] = pts
+    _check([int(l) for l in log2s], chunks, None, 3)
