@@ -2420,9 +2420,9 @@ __global__ void __launch_bounds__(32) k_selftest_wait(uint64_t* status, uint32_t
 // The reference runs one CTA per chunk and inserts values into a 64-slot shared
 // table in whatever order its threads arrive; the palette is the table's slot order.
 // Here chunks are cut into tiles of kPalTile voxels over the whole GPU: each tile
-// collects its distinct values with the first voxel index of each (every thread skips
-// the values it met last, the others go to a shared table), merges them into the
-// chunk's global table (value, first index by atomicMin), and one warp per chunk then
+// collects its distinct values with the first voxel index of each in a shared table,
+// merges them into the chunk's global table (value, first index by atomicMin; a chunk of
+// one tile stores them), and one warp per chunk then
 // inserts the values in order of
 // first occurrence into the reference's 64-slot table (same hash, linear probing)
 // to lay out the palette: the order the reference produces when its inserts arrive
@@ -2476,38 +2476,75 @@ __device__ __forceinline__ bool pal_insert(uint32_t* vals, uint32_t* firsts, uin
 
 // A step's kPalPer rows of kBlock attributes, all loads in flight. A block takes four
 // steps, since its look-ups before the first and its merge after the last are round
-// trips: scan + pack of 200 M attributes in 256 chunks take 691 / 614 / 568 us a call with
-// one / two / four (1208 when every row went through match_any, which costs some hundred
-// cycles where a row holds more than a few values, and every word's 8 attributes through
-// 16 comparisons each). Now the kernels take 180 and 221 us: the attributes' 0.8 GB are
-// 125 us at the copy rate, the pack writes another 0.25 GB.
+// trips: scan + pack of 200 M attributes in 256 chunks took 691 / 614 / 568 us a call with
+// one / two / four.
 constexpr uint32_t kPalStep = kPalTile / kPalSteps, kPalPer = kPalStep / kBlock;
+constexpr uint32_t kPalGroup = 4;  // rows looked up together
 __device__ __forceinline__ void pal_load(const uint32_t* attrs, uint32_t n, uint32_t (&v)[kPalPer]) {
 #pragma unroll
     for (uint32_t k = 0; k < kPalPer; ++k) {
+        if (k % kPalGroup == 0 && k * kBlock >= n) break;  // (a small chunk's rows end here: nothing reads the others)
         const uint32_t i = k * kBlock + threadIdx.x;
         v[k] = i < n ? __ldg(attrs + i) : kPalEmpty;
     }
 }
 
+// The chunk of a tile, by the whole warp. Where every chunk has one tile it needs no search
+// (four round trips of it: 100,000 chunks of 100 voxels 720 -> 618 us a scan).
+__device__ __forceinline__ uint32_t pal_chunk(const PaletteDesc& p, uint32_t tile) {
+    return gridDim.x == p.count ? tile : warp_upper_index(p.tile_of, p.count + 1, tile);
+}
+
+// A block's own table of values and first voxels, larger than the chunk's so that most
+// values are in their home slot.
+constexpr uint32_t kPalFind = 256;
+static_assert(kPalFind == kBlock, "a slot per thread");
+__device__ __forceinline__ uint32_t pal_home(uint32_t v, uint32_t mult) { return (v * mult) >> 24; }
+constexpr uint32_t kPalMult = 0x9E3779B1u;
+__device__ __forceinline__ uint2 pal_slot(const uint2* tab, uint32_t s) {
+    uint2 e;
+    const unsigned at = static_cast<unsigned>(__cvta_generic_to_shared(tab + s));
+    asm volatile("ld.volatile.shared.v2.u32 {%0, %1}, [%2];" : "=r"(e.x), "=r"(e.y) : "r"(at));
+    return e;
+}
+// Whether the table did not have the value yet (or has no room left).
+__device__ __forceinline__ bool pal_note(uint2* tab, uint32_t v, uint32_t idx) {
+    uint32_t s = pal_home(v, kPalMult);
+    for (uint32_t probes = 0; probes < kPalFind; ++probes) {
+        uint2 e = pal_slot(tab, s);
+        bool fresh = false;
+        if (e.x == kPalEmpty) {
+            e.x = atomicCAS(&tab[s].x, kPalEmpty, v);
+            fresh = e.x == kPalEmpty;
+            if (fresh) e.x = v;
+        }
+        if (e.x == v) {
+            if (e.y > idx) atomicMin(&tab[s].y, idx);
+            return fresh;
+        }
+        s = (s + 1) & (kPalFind - 1);
+    }
+    return true;
+}
+
 __global__ void __launch_bounds__(kBlock) k_pal_collect(PaletteDesc p) {
     grid_dep_wait();
-    __shared__ uint32_t s_val[kPalSlots], s_first[kPalSlots], s_found, s_over;
+    __shared__ uint2 s_tab[kPalFind];
+    __shared__ uint32_t s_found, s_over, s_at;
     const uint32_t tile = blockIdx.x;
-    if (threadIdx.x < kPalSlots) {
-        s_val[threadIdx.x] = kPalEmpty;
-        s_first[threadIdx.x] = 0xFFFFFFFFu;
-    }
-    const uint32_t c = warp_upper_index(p.tile_of, p.count + 1, tile);
+    s_tab[threadIdx.x] = make_uint2(kPalEmpty, 0xFFFFFFFFu);
+    const uint32_t c = pal_chunk(p, tile);
     if (c >= p.count) return;
-    const uint32_t lo = __ldg(p.first + c) + (tile - __ldg(p.tile_of + c)) * kPalTile;
+    const uint32_t tile0 = __ldg(p.tile_of + c);
+    const bool alone = __ldg(p.tile_of + c + 1) - tile0 == 1;  // the chunk's only tile
+    const uint32_t lo = __ldg(p.first + c) + (tile - tile0) * kPalTile;
     // (differences: the tile's end may lie beyond 32 bits)
     const uint32_t hi = lo + min(__ldg(p.first + c + 1) - lo, kPalTile);
     // (a chunk that another tile found to hold too many values: nothing more to learn. Other
     // blocks set the flag meanwhile: one thread's read decides for the block)
     if (threadIdx.x == 0) {
-        s_found = 0;
-        s_over = *reinterpret_cast<volatile uint32_t*>(p.gflag + c);
+        s_found = s_at = 0;
+        s_over = alone ? 0u : *reinterpret_cast<volatile uint32_t*>(p.gflag + c);
     }
     __syncthreads();
     if (s_over != 0) return;
@@ -2518,46 +2555,64 @@ __global__ void __launch_bounds__(kBlock) k_pal_collect(PaletteDesc p) {
     };
     uint32_t v[kPalPer];
     pal_load(p.attrs + lo, hi - lo, v);
-    // A thread passes over the two values it met last. Of the others in a row of the warp
-    // each value is inserted once, by its lowest lane: a thread's rows and a row's lanes are
-    // in index order, so the smallest index of a value is among the inserted ones.
-    // (0xFFFFFFFF is the table's empty marker and never enters a palette, as in the
-    // reference.)
+    // Most voxels' values are the thread's last one again, or in the table's home slot with
+    // an index at least as small: one look-up, for kPalGroup rows together. Where a lane's is
+    // not, the lanes of its row note theirs side by side, the first of each run only.
+    // (0xFFFFFFFF is the tables' empty marker and never enters a palette, as in the reference.)
+    // Calls of a scan: 200 M attributes in runs 181 us (125 at the copy rate); 10,000 chunks
+    // of 3000 voxels that take 16 values in random order 148, 100 chunks of 10^6 168. (A row's
+    // values found by match_any: 762 / 487 / 1156 us; each noted by one lane after another
+    // unless it was one of the thread's last two: 218 / 2066 / 9930.)
     const unsigned lane = threadIdx.x & 31;
-    uint32_t last0 = kPalEmpty, last1 = kPalEmpty;
+    uint32_t last = kPalEmpty;
     for (uint32_t base = lo; base - lo < hi - lo; base += kPalStep) {
         if (base != lo) pal_load(p.attrs + base, hi - base, v);
+        bool stop = false;
 #pragma unroll
-        for (uint32_t k = 0; k < kPalPer; ++k) {
-            const uint32_t x = v[k];
-            const bool need = x != kPalEmpty && x != last0 && x != last1;
-            unsigned todo = __ballot_sync(kFull, need);
-            if (!todo) continue;
-            if (full()) break;
-            while (todo) {
-                const uint32_t lead = __ffs(todo) - 1;
-                todo &= ~__ballot_sync(kFull, x == __shfl_sync(kFull, x, lead));
-                bool fresh = false;
-                if (lane == lead && (!pal_insert(s_val, s_first, x, base + k * kBlock + threadIdx.x, &fresh) || fresh))
-                    atomicAdd(&s_found, 1u);
+        for (uint32_t k0 = 0; k0 < kPalPer; k0 += kPalGroup) {
+            if (stop || k0 * kBlock >= hi - base) continue;
+            bool need[kPalGroup], any = false, diff = false;
+#pragma unroll
+            for (uint32_t q = 0; q < kPalGroup; ++q) diff = diff || v[k0 + q] != last;
+            if (!__any_sync(kFull, diff)) continue;
+#pragma unroll
+            for (uint32_t q = 0; q < kPalGroup; ++q) {
+                const uint32_t x = v[k0 + q];
+                const uint2 e = pal_slot(s_tab, pal_home(x, kPalMult));
+                need[q] = x != kPalEmpty && (e.x != x || e.y > base + (k0 + q) * kBlock + threadIdx.x);
+                any = any || need[q];
             }
-            if (need) {
-                last1 = last0;
-                last0 = x;
+            last = v[k0 + kPalGroup - 1];
+            if (!__any_sync(kFull, any)) continue;
+#pragma unroll
+            for (uint32_t q = 0; q < kPalGroup; ++q) {
+                if (stop || !__any_sync(kFull, need[q])) continue;
+                stop = full();
+                if (stop) continue;
+                const uint32_t x = v[k0 + q], left = __shfl_up_sync(kFull, x, 1);
+                if (need[q] && (lane == 0 || left != x) &&
+                    pal_note(s_tab, x, base + (k0 + q) * kBlock + threadIdx.x))
+                    atomicAdd(&s_found, 1u);
+                __syncwarp();
             }
         }
-        if (full()) break;
+        if (stop || full()) break;
     }
     __syncthreads();
     if (s_found > kPalMax) {  // the chunk keeps its 32-bit attributes
         if (threadIdx.x == 0) atomicOr(p.gflag + c, 1u);
         return;
     }
-    if (threadIdx.x < kPalSlots && s_val[threadIdx.x] != kPalEmpty) {
-        bool fresh;
-        if (!pal_insert(p.gval + uint64_t(c) * kPalSlots, p.gfirst + uint64_t(c) * kPalSlots, s_val[threadIdx.x],
-                        s_first[threadIdx.x], &fresh))
-            atomicOr(p.gflag + c, 1u);
+    const uint2 e = s_tab[threadIdx.x];
+    if (e.x == kPalEmpty) return;
+    uint32_t *gval = p.gval + uint64_t(c) * kPalSlots, *gfirst = p.gfirst + uint64_t(c) * kPalSlots;
+    bool fresh;
+    if (alone) {  // (the slots' order does not matter to k_pal_layout)
+        const uint32_t at = atomicAdd(&s_at, 1u);
+        gval[at] = e.x;
+        gfirst[at] = e.y;
+    } else if (!pal_insert(gval, gfirst, e.x, e.y, &fresh)) {
+        atomicOr(p.gflag + c, 1u);
     }
 }
 
@@ -2612,19 +2667,31 @@ __global__ void __launch_bounds__(kBlock) k_pal_layout(PaletteDesc p) {
     if (lane == 0) p.counts[c] = n;
 }
 
-// palette.zig pack: rows of 32 voxels per warp; a voxel's index comes from a table of the
-// palette (or is the thread's last one again), 8 lanes join theirs to a word.
-__global__ void __launch_bounds__(kBlock) k_pal_pack(PaletteDesc p) {
+// palette.zig pack: rows of 32 voxels per warp, 8 lanes join their indices to a word. A
+// voxel's index comes from a table in which every palette entry has a slot of its own (a
+// multiplier spreads 16 entries over 256 slots with better than 6 in 10, and there are
+// kPalTries of them), so a look-up is one load and one comparison, whatever the order of the
+// values. Where none does, the entries are compared one after another. Calls of a pack: 200 M
+// attributes in runs 243 us, 10,000 chunks of 3000 voxels in random order of 16 values 102;
+// with 16 comparisons each 411 / 139, with a probed table and each thread's last value 242 /
+// 216. 6 blocks per SM (40 registers) rather than 4 (64): 261 -> 243.
+constexpr uint32_t kPalTries = 8;
+__host__ __device__ __forceinline__ uint32_t pal_mult(uint32_t t) { return kPalMult + t * 0x3C6EF372u; }  // (odd)
+
+__global__ void __launch_bounds__(kBlock, 6) k_pal_pack(PaletteDesc p) {
     grid_dep_wait();
-    __shared__ uint32_t s_val[kPalSlots], s_ix[kPalSlots], s_none;
+    __shared__ uint2 s_map[kPalFind];     // value, index
+    __shared__ uint32_t s_pal[kPalMax], s_mult;
     const uint32_t tile = blockIdx.x;
-    const uint32_t c = warp_upper_index(p.tile_of, p.count + 1, tile);
+    const uint32_t c = pal_chunk(p, tile);
     if (c >= p.count) return;
     const uint32_t lo = __ldg(p.first + c), n = __ldg(p.first + c + 1) - lo;
     const uint32_t t0 = (tile - __ldg(p.tile_of + c)) * kPalTile;  // first voxel of the tile within the chunk
     const uint32_t t1 = t0 + min(n - t0, kPalTile);
     uint32_t* out = p.pool + __ldg(p.dst + c);
     const bool raw = __ldg(p.counts + c) == kPalOverflow;
+    uint32_t entry = 0;
+    if (threadIdx.x < kPalMax) entry = p.palettes[uint64_t(c) * kPalMax + threadIdx.x];
     uint32_t v[kPalPer];
     pal_load(p.attrs + lo + t0, t1 - t0, v);
     if (raw) {
@@ -2636,43 +2703,60 @@ __global__ void __launch_bounds__(kBlock) k_pal_pack(PaletteDesc p) {
         }
         return;
     }
-    if (threadIdx.x < kPalSlots) {
-        s_val[threadIdx.x] = kPalEmpty;
-        s_ix[threadIdx.x] = 0xFFFFFFFFu;
-    }
-    if (threadIdx.x == 0) s_none = kPalMax;
+    s_map[threadIdx.x] = make_uint2(0u, 0xFFFFFFFFu);  // (a free slot: index -1)
     __syncthreads();
-    if (threadIdx.x < kPalMax) {
-        const uint32_t x = p.palettes[uint64_t(c) * kPalMax + threadIdx.x];
-        if (t0 == 0) out[threadIdx.x] = x;
-        // of equal entries the first; the table's empty marker (in a caller's own palette)
-        // has its index beside the table
-        bool fresh;
-        if (x != kPalEmpty) pal_insert(s_val, s_ix, x, threadIdx.x, &fresh);
-        else atomicMin(&s_none, threadIdx.x);
+    if (threadIdx.x < 32) {
+        const unsigned lane = threadIdx.x;
+        if (lane < kPalMax) {
+            s_pal[lane] = entry;
+            if (t0 == 0) out[lane] = entry;
+        }
+        // (the padding repeats the first entry)
+        const uint32_t entry0 = __shfl_sync(kFull, entry, 0);
+        const bool set = lane == 0 || (lane < kPalMax && entry != entry0);
+        uint32_t mult = 0;
+        for (uint32_t t = 0; t < kPalTries && mult == 0; ++t) {
+            const uint32_t m = pal_mult(t);
+            uint2* slot = s_map + pal_home(entry, m);
+            const uint32_t old = set ? atomicCAS(&slot->y, 0xFFFFFFFFu, lane) : 0xFFFFFFFFu;
+            __syncwarp();
+            // (another entry of the same value: the first one counts)
+            const uint32_t other = __shfl_sync(kFull, entry, old & 31);
+            const bool taken = old != 0xFFFFFFFFu, same = taken && other == entry;
+            if (same) atomicMin(&slot->y, lane);
+            __syncwarp();
+            if (!__any_sync(kFull, taken && !same)) {
+                if (set) slot->x = entry;
+                mult = m;
+            } else {
+                if (set) slot->y = 0xFFFFFFFFu;
+            }
+            __syncwarp();
+        }
+        if (lane == 0) s_mult = mult;
     }
     __syncthreads();
-    const uint32_t none = s_none < kPalMax ? s_none : 0u;
-    uint32_t last = kPalEmpty, ix = none;
+    const uint32_t mult = s_mult;
     for (uint32_t base = t0; base - t0 < t1 - t0; base += kPalStep) {
         if (base != t0) pal_load(p.attrs + lo + base, t1 - base, v);
 #pragma unroll
         for (uint32_t k = 0; k < kPalPer; ++k) {
-            const uint32_t i = base + k * kBlock + threadIdx.x;
-            if (v[k] != last) {
-                // (a value outside the palette has index 0)
-                last = v[k];
-                ix = last == kPalEmpty ? none : 0u;
-                uint32_t s = pal_hash(last) & (kPalSlots - 1);
-                for (uint32_t key; last != kPalEmpty && (key = s_val[s]) != kPalEmpty; s = (s + 1) & (kPalSlots - 1))
-                    if (key == last) { ix = s_ix[s]; break; }
+            if (k % kPalGroup == 0 && k * kBlock >= t1 - base) break;
+            const uint32_t x = v[k];
+            uint32_t ix = 0;  // (a value outside the palette has index 0)
+            if (mult != 0) {
+                const uint2 e = s_map[pal_home(x, mult)];
+                ix = e.x == x && e.y != 0xFFFFFFFFu ? e.y : 0u;
+            } else {
+                for (uint32_t q = kPalMax; q-- > 0;)
+                    if (s_pal[q] == x) ix = q;  // the first equal entry
             }
             const bool in = k * kBlock + threadIdx.x < t1 - base;
             uint32_t word = in ? ix << ((threadIdx.x & 7) * 4) : 0u;
             word |= __shfl_xor_sync(kFull, word, 1);
             word |= __shfl_xor_sync(kFull, word, 2);
             word |= __shfl_xor_sync(kFull, word, 4);
-            if ((threadIdx.x & 7) == 0 && in) out[kPalMax + i / 8] = word;
+            if ((threadIdx.x & 7) == 0 && in) out[kPalMax + (base + k * kBlock + threadIdx.x) / 8] = word;
         }
     }
 }

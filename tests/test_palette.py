@@ -179,3 +179,43 @@ def test_palette_of_the_last_voxel_indices(sizes):
     gpu_build.palette_pack(addr, first, pal, cnt, dst, pool)
     opool = orc.palette_pack(attrs, ofirst, opal, ocnt, dst, total)
     assert np.array_equal(pool.cpu().numpy().view(np.uint32)[:total], opool)
+
+
+# The pack's table gives every palette entry a slot of its own, by the first of eight
+# multipliers that does; these values share a slot under each of them. Palettes of the
+# caller's may repeat entries and hold the table's empty marker; voxels outside have index 0.
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", ["spread", "clash", "clash16", "repeats", "marker", "zero"])
+def test_palette_pack_tables(kind):
+    import torch
+    from pyrit_b200 import gpu_build
+    from gpu_helpers import dev
+    rng = np.random.default_rng(len(kind))
+    vals = [int(v) for v in rng.integers(1, 1 << 32, 16, dtype=np.uint64)]
+    if kind.startswith("clash"):
+        for t in range(8):
+            m = (0x9E3779B1 + t * 0x3C6EF372) & 0xFFFFFFFF
+            vals[t + 1] = (vals[t] + pow(m, -1, 1 << 32)) & 0xFFFFFFFF
+            assert (vals[t] * m & 0xFFFFFFFF) >> 24 == (vals[t + 1] * m & 0xFFFFFFFF) >> 24
+        if kind == "clash":
+            vals[9:] = [vals[0]] * 7
+    if kind == "repeats":
+        vals = [vals[i] for i in (0, 1, 2, 1, 3, 2, 0, 4, 4, 4, 5, 1, 6, 6, 0, 0)]
+    if kind == "marker":
+        vals[5] = vals[9] = OVER
+    if kind == "zero":
+        vals[3] = 0
+    pal = np.array([vals, vals[::-1]], np.uint32)
+    outside = rng.integers(1, 1 << 32, 5, dtype=np.uint64).astype(np.uint32)
+    pool = np.concatenate([pal[0], outside, np.array([0, OVER], np.uint32)])
+    attrs = rng.choice(pool, 40_000).astype(np.uint32)
+    first = np.array([0, 20_001, 40_000], np.uint32)
+    cnt = np.array([16, 16], np.uint32)
+    dst, total = orc.palette_layout(first, cnt)
+    out = torch.zeros(total, dtype=torch.int32, device="cuda")
+    gpu_build.palette_pack(dev(attrs), first, dev(pal), cnt, dst, out)
+    want = orc.palette_pack(attrs, first, pal, cnt, dst, total)
+    assert np.array_equal(out.cpu().numpy().view(np.uint32), want)
+    # the same values found by a scan
+    if kind in ("spread", "clash", "clash16"):
+        _check_against_oracle(np.resize(pal[0], 30_000), dev(np.resize(pal[0], 30_000)), np.array([0, 17, 30_000], np.uint32))
