@@ -537,9 +537,14 @@ __global__ void __launch_bounds__(NT, PYRB_SORT_MIN_BLOCKS * kBlock / NT) k_sort
 // ---------------------------------------------------------------------------
 
 // Slots of a dedup table for `count` items: what the load factor asks for, at most the
-// allocated `bound` (sized by the largest count that the input could have).
+// allocated `bound` (sized by the largest count that the input could have). Small tables take
+// four times that: their inserts wait for the longest probe sequence, a round trip a slot, and
+// a megabyte costs nothing to clear (20,000 voxels in a corner of a 2^10 volume 162 -> 156 us a
+// call, 159 when all of the bound was used; 256^3 to 128^3 147 -> 144). Up to 2^16 slots asked
+// for instead of 2^14: nothing more, and 1 to 2 % on larger levels lost to the clearing.
 __device__ __forceinline__ uint32_t table_slots(const BuildDesc& d, uint32_t count, uint32_t bound) {
-    const uint64_t need = (uint64_t(count) * 100 + d.load_pct - 1) / d.load_pct;
+    uint64_t need = (uint64_t(count) * 100 + d.load_pct - 1) / d.load_pct;
+    if (need <= (1u << 14)) need *= 4;
     if (need >= bound) return bound;
     return need <= 1024 ? min(1024u, bound) : min(1u << (32 - __clz(uint32_t(need) - 1)), bound);
 }

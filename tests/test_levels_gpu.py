@@ -92,3 +92,19 @@ def test_order_of_the_old_voxels(order, n_new):
     finally:
         gpu_build.set_tuning(0, 0, 50, 0)
     assert_same_build(g, orc.gb_build(log2, 4, ed, old_keys=keys, old_vals=vals), label=order)
+
+
+@pytest.mark.parametrize("load", [25, 50, 90])
+@pytest.mark.parametrize("n", [4096 * 4, 8192, 8193, 14745, 14747])
+def test_table_sizes(n, load):
+    """Bricks and parents at the counts where their tables stop taking four times the slots
+    that the load factor asks for (2^14 slots), one voxel each and all of them different."""
+    from pyrit_b200 import gpu_build
+    rng = np.random.default_rng(n)
+    pts = _bricks(rng, 9, n, 1)
+    gpu_build.set_tuning(0, 0, load, 0)
+    try:
+        g = gpu_build.build(9, 5, dev(pts)).download()
+    finally:
+        gpu_build.set_tuning(0, 0, 50, 0)
+    assert_same_build(g, orc.gb_build(9, 5, pts), label=f"{n} {load}")
